@@ -28,26 +28,68 @@
 #include "../../include/rfmanta_b200.h"
 #include "rq_batch.h"
 #include "rq_scene.h"
-#include "rq_traverse.cuh"
+#include "rq_wide.cuh"
 
 namespace rq {
 
-// Resets a lane's traversal stack: a RegStack over the thread's shared
+// The binary walk over either stack: a RegStack over the thread's shared
 // column, or a SplitStack whose first A.stack_depth entries sit there and
 // whose deeper ones go to the thread's entries of the overflow area.
-template <int R>
-__device__ __forceinline__ void reset_stack(RegStack<R>& st, int2* smem, const BatchArgs&) {
-  st.init(smem + threadIdx.x, blockDim.x);
-}
-__device__ __forceinline__ void reset_stack(SplitStack& st, int2* smem, const BatchArgs& A) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  st.init(smem + threadIdx.x, A.stack_depth, A.ovf + g);
-}
+template <int KIND_, int R, bool STATS_, bool SPLIT>
+struct BatchBinary {
+  static constexpr int KIND = KIND_;
+  static constexpr bool STATS = STATS_, WIDE = false;
+  typename std::conditional<SPLIT, SplitStack, RegStack<R>>::type st;
+  Counts cnt;
+  static __device__ __forceinline__ void reset(RegStack<R>& s, int2* smem, const BatchArgs&) {
+    s.init(smem + threadIdx.x, blockDim.x);
+  }
+  static __device__ __forceinline__ void reset(SplitStack& s, int2* smem, const BatchArgs& A) {
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    s.init(smem + threadIdx.x, A.stack_depth, A.ovf + g);
+  }
+  __device__ __forceinline__ void init(int2* smem, const BatchArgs& A) { reset(st, smem, A); }
+  __device__ __forceinline__ void start(const DevScene& S, Ray& r, bool any, Hit& h, int& ref,
+                                        int2* smem, const BatchArgs& A) {
+    int sp0;
+    start_ray(S, r, h, ref, sp0);
+    reset(st, smem, A);
+    if (STATS) cnt.boxes += 1;
+  }
+  // Work is ordered scene by scene, closest-hit batches before any-hit ones,
+  // so a warp's busy lanes almost always share the query kind: the step is
+  // then compiled for that kind (the per-lane form only where kinds meet).
+  __device__ __forceinline__ void step(const DevScene& S, Ray& r, Hit& h, bool any, bool live,
+                                       int vote, int& ref) {
+    const unsigned any_m = __ballot_sync(0xffffffffu, live && any);
+    const unsigned clo_m = __ballot_sync(0xffffffffu, live && !any);
+    if (!live) return;
+    if (any_m == 0u)
+      step_dyn<KIND, R, STATS>(S, r, h, ref, st, false, &cnt);
+    else if (clo_m == 0u)
+      step_dyn<KIND, R, STATS>(S, r, h, ref, st, true, &cnt);
+    else
+      step_dyn<KIND, R, STATS>(S, r, h, ref, st, any, &cnt);
+  }
+};
 
-// SPLIT: the stack is a SplitStack with a short shared column, and
+template <int KIND_>
+struct BatchWide : WideWalk<KIND_> {
+  __device__ __forceinline__ void init(int2* smem, const BatchArgs&) {
+    WideWalk<KIND_>::init(smem);
+  }
+  __device__ __forceinline__ void start(const DevScene& S, Ray& r, bool any, Hit& h, int& ref,
+                                        int2*, const BatchArgs&) {
+    WideWalk<KIND_>::start(S, r, any, h, ref);
+  }
+};
+
+constexpr int kBatchVote = 16;  // wide walk (rq_wide.cuh)
+
+// SPLIT: the walk's stack is a SplitStack with a short shared column, and
 // registers are held to 48 per thread (five 256-thread blocks per SM), so
 // more warps are resident to hide the traversal's dependent loads.
-template <int KIND, int R, bool STATS, bool SPLIT>
+template <class Walk, bool SPLIT>
 __global__ void __launch_bounds__(256, SPLIT ? 5 : 1) batch_kernel(BatchArgs A) {
   extern __shared__ int2 smem[];
   __shared__ DevScene sm_scenes[kMaxBatchScenes];
@@ -55,8 +97,8 @@ __global__ void __launch_bounds__(256, SPLIT ? 5 : 1) batch_kernel(BatchArgs A) 
   __syncthreads();
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lt = (1u << lane) - 1u;
-  typename std::conditional<SPLIT, SplitStack, RegStack<R>>::type st;
-  reset_stack(st, smem, A);
+  Walk walk;
+  walk.init(smem, A);
   // warp-uniform chunk state
   int w_batch = 0, w_next = 0, w_end = 0;
   bool exhausted = false;
@@ -66,7 +108,6 @@ __global__ void __launch_bounds__(256, SPLIT ? 5 : 1) batch_kernel(BatchArgs A) 
   Ray r;
   Hit h;
   int ref = kDone;
-  Counts cnt;
   for (;;) {
     const unsigned idle = __ballot_sync(0xffffffffu, my_ray < 0);
     const unsigned busy = ~idle;
@@ -105,10 +146,7 @@ __global__ void __launch_bounds__(256, SPLIT ? 5 : 1) batch_kernel(BatchArgs A) 
             r.inv[c] = fdiv(1.f, r.d[c]);
           }
           r.minT = __ldg(B.tmax + my_ray);
-          int sp0;
-          start_ray(sm_scenes[B.scene], r, h, ref, sp0);
-          reset_stack(st, smem, A);
-          if (STATS) cnt.boxes += 1;
+          walk.start(sm_scenes[B.scene], r, B.any != 0, h, ref, smem, A);
         }
         const unsigned taken = __ballot_sync(0xffffffffu, take);
         need &= ~taken;
@@ -116,105 +154,67 @@ __global__ void __launch_bounds__(256, SPLIT ? 5 : 1) batch_kernel(BatchArgs A) 
       }
     }
     if (exhausted && __all_sync(0xffffffffu, my_ray < 0)) break;
-    // Work is ordered scene by scene, closest-hit batches before any-hit
-    // ones, so a warp's busy lanes almost always share the query kind: the
-    // step is then compiled for that kind (the per-lane form only where
-    // kinds meet).
-    const bool stepping = my_ray >= 0 && ref != kDone;
-    const bool my_any = (my_tag & 1) != 0;
-    const int my_scene = (my_tag >> 1) & 31;
-    const unsigned any_m = __ballot_sync(0xffffffffu, stepping && my_any);
-    const unsigned clo_m = __ballot_sync(0xffffffffu, stepping && !my_any);
-    if (my_ray >= 0) {
-      if (stepping) {
-        // the lane's scene descriptor copied to registers: the step's stack
-        // stores go to shared memory too, and a descriptor read from there
-        // would be read again after every store
-        DevScene S;
-        S.nodes = sm_scenes[my_scene].nodes;
-        S.tris = sm_scenes[my_scene].tris;
-        if (any_m == 0u)
-          step_dyn<KIND, R, STATS>(S, r, h, ref, st, false, &cnt);
-        else if (clo_m == 0u)
-          step_dyn<KIND, R, STATS>(S, r, h, ref, st, true, &cnt);
-        else
-          step_dyn<KIND, R, STATS>(S, r, h, ref, st, my_any, &cnt);
-      }
-      if (ref == kDone) {
-        const BatchDesc& B = A.batches[my_tag >> 6];
-        if (B.t) B.t[my_ray] = h.t;
-        if (B.prim) B.prim[my_ray] = h.id;
-        if (B.u) B.u[my_ray] = h.u;
-        if (B.v) B.v[my_ray] = h.v;
-        my_ray = -1;
-      }
+    // the lane's scene descriptor copied to registers: the step's stack
+    // stores go to shared memory too, and a descriptor read from there
+    // would be read again after every store
+    const DevScene S = walk_scene<Walk>(sm_scenes[(my_tag >> 1) & 31]);
+    walk.step(S, r, h, (my_tag & 1) != 0, my_ray >= 0 && ref != kDone, kBatchVote, ref);
+    if (my_ray >= 0 && ref == kDone) {
+      const BatchDesc& B = A.batches[my_tag >> 6];
+      if (B.t) B.t[my_ray] = h.t;
+      if (B.prim) B.prim[my_ray] = h.id;
+      if (B.u) B.u[my_ray] = h.u;
+      if (B.v) B.v[my_ray] = h.v;
+      my_ray = -1;
     }
   }
-  if (STATS) {
-    atomicAdd(&A.stats[0], (unsigned long long)cnt.boxes);
-    atomicAdd(&A.stats[1], (unsigned long long)cnt.tris);
+  if (Walk::STATS) {
+    atomicAdd(&A.stats[0], (unsigned long long)walk.cnt.boxes);
+    atomicAdd(&A.stats[1], (unsigned long long)walk.cnt.tris);
   }
 }
 
-template <int KIND, int R, bool STATS, bool SPLIT = false>
-static cudaError_t batch_go(bool launch, int grid, int block, size_t smem, const BatchArgs& A,
-                            cudaStream_t st, const void** fn) {
-  if (fn) *fn = (const void*)batch_kernel<KIND, R, STATS, SPLIT>;
-  if (launch) batch_kernel<KIND, R, STATS, SPLIT><<<grid, block, smem, st>>>(A);
-  return launch ? cudaGetLastError() : cudaSuccess;
-}
-
-// Resolves (triangle kind, register stack, statistics) to one kernel and
-// either returns its address or launches it; reg = kSplitStack selects the
-// split-stack kernel.
+// The kernel of a plan: the wide walk, or the binary one with `reg` register
+// stack entries (kSplitStack: its split stack).
 constexpr int kSplitStack = -1;
-template <int KIND>
-static cudaError_t batch_dispatch_kind(int reg, bool stats, bool launch, int grid, int block,
-                                       size_t smem, const BatchArgs& A, cudaStream_t st,
-                                       const void** fn) {
+template <int KIND, bool STATS>
+static const void* batch_binary_fn(int reg) {
   switch (reg) {
-    case kSplitStack:
-      return stats ? batch_go<KIND, 0, true, true>(launch, grid, block, smem, A, st, fn)
-                   : batch_go<KIND, 0, false, true>(launch, grid, block, smem, A, st, fn);
-    case 1:
-      return stats ? batch_go<KIND, 1, true>(launch, grid, block, smem, A, st, fn)
-                   : batch_go<KIND, 1, false>(launch, grid, block, smem, A, st, fn);
-    case 2:
-      return stats ? batch_go<KIND, 2, true>(launch, grid, block, smem, A, st, fn)
-                   : batch_go<KIND, 2, false>(launch, grid, block, smem, A, st, fn);
-    case 4:
-      return stats ? batch_go<KIND, 4, true>(launch, grid, block, smem, A, st, fn)
-                   : batch_go<KIND, 4, false>(launch, grid, block, smem, A, st, fn);
-    default:
-      return stats ? batch_go<KIND, 0, true>(launch, grid, block, smem, A, st, fn)
-                   : batch_go<KIND, 0, false>(launch, grid, block, smem, A, st, fn);
+    case kSplitStack: return (const void*)batch_kernel<BatchBinary<KIND, 0, STATS, true>, true>;
+    case 1: return (const void*)batch_kernel<BatchBinary<KIND, 1, STATS, false>, false>;
+    case 2: return (const void*)batch_kernel<BatchBinary<KIND, 2, STATS, false>, false>;
+    case 4: return (const void*)batch_kernel<BatchBinary<KIND, 4, STATS, false>, false>;
+    default: return (const void*)batch_kernel<BatchBinary<KIND, 0, STATS, false>, false>;
   }
 }
-
-static cudaError_t batch_dispatch(int kind, int reg, bool stats, bool launch, int grid,
-                                  int block, size_t smem, const BatchArgs& A, cudaStream_t st,
-                                  const void** fn) {
+static const void* batch_fn(int kind, int reg, bool wide, bool stats) {
   if (kind == kWald)
-    return batch_dispatch_kind<kWald>(reg, stats, launch, grid, block, smem, A, st, fn);
-  return batch_dispatch_kind<kKS>(reg, stats, launch, grid, block, smem, A, st, fn);
+    return wide    ? (const void*)batch_kernel<BatchWide<kWald>, false>
+           : stats ? batch_binary_fn<kWald, true>(reg)
+                   : batch_binary_fn<kWald, false>(reg);
+  return wide    ? (const void*)batch_kernel<BatchWide<kKS>, false>
+         : stats ? batch_binary_fn<kKS, true>(reg)
+                 : batch_binary_fn<kKS, false>(reg);
 }
 
-cudaError_t launch_batch(int tri_kind, int reg_stack, const BatchArgs& A, int grid, int block,
-                         size_t smem, cudaStream_t st) {
-  const void* f = nullptr;
-  batch_dispatch(tri_kind, reg_stack, A.stats != nullptr, false, 0, 0, 0, A, nullptr, &f);
+static cudaError_t batch_launch(const void* f, int grid, int block, size_t smem,
+                                const BatchArgs& A, cudaStream_t st) {
+  void* args[] = {(void*)&A};
+  return cudaLaunchKernel(f, dim3(grid), dim3(block), args, smem, st);
+}
+
+cudaError_t launch_batch(int tri_kind, int reg_stack, bool wide, const BatchArgs& A, int grid,
+                         int block, size_t smem, cudaStream_t st) {
+  const void* f = batch_fn(tri_kind, reg_stack, wide, A.stats != nullptr);
   // static shared memory (the scene table) counts against the default 48 KB
   // too, so the dynamic size is always declared
   if (smem > 0)
     cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  return batch_dispatch(tri_kind, reg_stack, A.stats != nullptr, true, grid, block, smem, A, st,
-                        nullptr);
+  return batch_launch(f, grid, block, smem, A, st);
 }
 
-int batch_blocks_per_sm(int tri_kind, int reg_stack, int block, size_t smem) {
-  const void* f = nullptr;
-  BatchArgs A{};
-  batch_dispatch(tri_kind, reg_stack, false, false, 0, 0, 0, A, nullptr, &f);
+int batch_blocks_per_sm(int tri_kind, int reg_stack, bool wide, int block, size_t smem) {
+  const void* f = batch_fn(tri_kind, reg_stack, wide, false);
   if (smem > 0)
     cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int b = 0;
@@ -247,6 +247,7 @@ struct rq_batch_plan {
   std::vector<uint64_t> generations;
   std::vector<rq::DevScene> host_scenes;
   int stack_depth = 1;
+  bool wide = false;  // the captured kernel walks wide nodes
   int num_sms = 148;
   ~rq_batch_plan() {
     if (exec) cudaGraphExecDestroy(exec);
@@ -291,11 +292,12 @@ int capture_plan(rq_batch_plan* p) {
   const int reg = split ? kSplitStack : cfg.reg_stack;
   A.stack_depth = split ? std::min(cfg.smem_entries, p->stack_depth) : p->stack_depth;
   // the shared-memory column holds what the register entries do not
-  p->smem = (size_t)std::max(1, A.stack_depth - (split ? 0 : cfg.reg_stack)) *
-            cfg.block_threads * sizeof(int2);
-  const bool stats = A.stats != nullptr;
-  const void* f = nullptr;
-  batch_dispatch(p->tri_kind, reg, stats, false, 0, 0, 0, A, nullptr, &f);
+  // (register entries, a split stack, another record order and counted tests
+  // are the binary walk's; node_layout clears the descriptors' wide nodes)
+  p->wide = !split && cfg.reg_stack == 0 && A.stats == nullptr;
+  for (const DevScene& d : p->host_scenes) p->wide = p->wide && d.wide;
+  p->smem = stack_bytes(A.stack_depth, cfg.block_threads, p->wide, split ? 0 : cfg.reg_stack);
+  const void* f = batch_fn(p->tri_kind, reg, p->wide, A.stats != nullptr);
   if (p->smem > 0 &&
       cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem) !=
           cudaSuccess)
@@ -333,8 +335,7 @@ int capture_plan(rq_batch_plan* p) {
   cudaError_t e = cudaStreamBeginCapture(p->cap_stream, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
     cudaMemsetAsync(p->d_counter, 0, sizeof(int), p->cap_stream);
-    batch_dispatch(p->tri_kind, reg, stats, true, p->grid, cfg.block_threads, p->smem, A,
-                   p->cap_stream, nullptr);
+    batch_launch(f, p->grid, cfg.block_threads, p->smem, A, p->cap_stream);
     e = cudaStreamEndCapture(p->cap_stream, &p->graph);
   }
   if (e == cudaSuccess && split) {
@@ -508,10 +509,13 @@ int rq_batch_plan_launch(rq_batch_plan* plan, void* stream) {
   if (changed) {
     int depth = 1;
     for (const rq::DevScene& d : plan->host_scenes) depth = std::max(depth, d.depth);
-    if (depth > plan->stack_depth) {
-      // a deeper tree: a larger stack, captured again (after the launches
-      // already queued, which still use the old graph)
-      plan->stack_depth = depth;
+    bool wide = plan->wide;
+    for (const rq::DevScene& d : plan->host_scenes) wide = wide && d.wide;
+    if (depth > plan->stack_depth || wide != plan->wide) {
+      // a deeper tree, or one without wide nodes: a larger stack or the
+      // binary walk, captured again (after the launches already queued, which
+      // still use the old graph)
+      plan->stack_depth = std::max(depth, plan->stack_depth);
       const int rc = capture_plan(plan);
       if (rc != RQ_OK) return rc;
     }

@@ -45,9 +45,10 @@ struct BatchArgs {
 };
 
 // The persistent batched kernel (counter must be zero) with `reg_stack`
-// register entries (0, 1, 2, 4) and `smem` bytes of stack per block.
-cudaError_t launch_batch(int tri_kind, int reg_stack, const BatchArgs& A, int grid, int block,
+// register entries (0, 1, 2, 4) or, with 0 and `wide`, the wide walk (every
+// scene's tree has wide nodes), and `smem` bytes of stack per block.
+cudaError_t launch_batch(int tri_kind, int reg_stack, bool wide, const BatchArgs& A, int grid, int block,
                          size_t smem, cudaStream_t st);
-int batch_blocks_per_sm(int tri_kind, int reg_stack, int block, size_t smem);
+int batch_blocks_per_sm(int tri_kind, int reg_stack, bool wide, int block, size_t smem);
 
 }  // namespace rq

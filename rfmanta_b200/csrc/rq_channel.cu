@@ -50,7 +50,7 @@
 
 #include "../../include/rfmanta_b200.h"
 #include "rq_scene.h"
-#include "rq_traverse.cuh"
+#include "rq_wide.cuh"
 
 namespace rq {
 
@@ -131,37 +131,45 @@ __device__ __forceinline__ unsigned long long now_ns() {
   return t;
 }
 
+constexpr int kChanVote = 12;  // as kClosestVote (rq_trace.cu)
+
 // Traces packet rays [0, n) of one slot: per ray two float4 in `in`
 // (origin, minT; direction, 0) and one float4 out (t, triangle id bits, u,
 // v), so a ray costs two loads and one store across PCIe.  Rays are read
 // with ld.cv (the host rewrites them for every request).
-template <int KIND, bool ANY>
+template <class Walk>
 __device__ __forceinline__ void serve_rays(const DevScene& S, const float4* in, float4* out,
-                                           int n, int2* stk) {
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const float4 a = __ldcv(in + 2 * i);
-    const float4 b = __ldcv(in + 2 * i + 1);
+                                           int n, bool any, Walk& walk) {
+  // whole warps step together: a warp stays while any of its lanes has a ray
+  for (int i = threadIdx.x; (i & ~31) < n; i += blockDim.x) {
     Ray r;
-    r.o[0] = a.x;
-    r.o[1] = a.y;
-    r.o[2] = a.z;
-    r.minT = a.w;
-    r.d[0] = b.x;
-    r.d[1] = b.y;
-    r.d[2] = b.z;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) r.inv[c] = fdiv(1.f, r.d[c]);  // RayPacket.cc:106-110
     Hit h;
-    int ref, sp;
-    start_ray(S, r, h, ref, sp);
-    while (ref != kDone) step<KIND, ANY>(S, r, h, ref, sp, stk, blockDim.x);
-    out[i] = make_float4(h.t, __int_as_float(h.id), h.u, h.v);
+    int ref = kDone;
+    if (i < n) {
+      const float4 a = __ldcv(in + 2 * i);
+      const float4 b = __ldcv(in + 2 * i + 1);
+      r.o[0] = a.x;
+      r.o[1] = a.y;
+      r.o[2] = a.z;
+      r.minT = a.w;
+      r.d[0] = b.x;
+      r.d[1] = b.y;
+      r.d[2] = b.z;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) r.inv[c] = fdiv(1.f, r.d[c]);  // RayPacket.cc:106-110
+      walk.start(S, r, any, h, ref);
+    }
+    while (__any_sync(0xffffffffu, ref != kDone))
+      walk.step(S, r, h, any, ref != kDone, kChanVote, ref);
+    if (i < n) out[i] = make_float4(h.t, __int_as_float(h.id), h.u, h.v);
   }
 }
 
-template <int KIND>
+template <class Walk>
 __global__ void __launch_bounds__(kChanThreads) channel_kernel(ChanArgs A) {
   extern __shared__ int2 stk[];
+  Walk walk;
+  walk.init(stk);
   __shared__ unsigned s_req;
   __shared__ int s_cmd, s_n, s_any;
   __shared__ unsigned long long s_t;
@@ -226,9 +234,7 @@ __global__ void __launch_bounds__(kChanThreads) channel_kernel(ChanArgs A) {
     const int cmd = s_cmd;
     if (cmd == 2) break;
     if (cmd == 1) {
-      int2* col = stk + threadIdx.x;
-      if (s_any) serve_rays<KIND, true>(A.S, in, out, s_n, col);
-      else serve_rays<KIND, false>(A.S, in, out, s_n, col);
+      serve_rays(A.S, in, out, s_n, s_any != 0, walk);
       // the CTA's hit stores are ordered before thread 0's release of
       // `done` by the barrier; the release at system scope is cumulative
       __syncthreads();
@@ -333,9 +339,13 @@ int relaunch(rq_channel* ch, unsigned seen_epoch) {
   A.max_rays = ch->max_rays;
   A.idle_ns = ch->idle_ns;
   A.life_ns = ch->life_ns;
-  const size_t smem = (size_t)std::max(1, A.S.depth) * kChanThreads * sizeof(int2);
-  const void* f = s->tri_kind == kWald ? (const void*)channel_kernel<kWald>
-                                       : (const void*)channel_kernel<kKS>;
+  const bool wide = A.S.wide != nullptr;
+  const size_t smem = stack_bytes(A.S.depth, kChanThreads, wide);
+  const void* f = s->tri_kind == kWald
+                      ? (wide ? (const void*)channel_kernel<WideWalk<kWald>>
+                              : (const void*)channel_kernel<BinaryWalk<kWald, false, 0>>)
+                      : (wide ? (const void*)channel_kernel<WideWalk<kKS>>
+                              : (const void*)channel_kernel<BinaryWalk<kKS, false, 0>>);
   if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
     return cfail(RQ_ERR_CAPACITY, "channel: traversal stack does not fit in shared memory");
@@ -343,11 +353,8 @@ int relaunch(rq_channel* ch, unsigned seen_epoch) {
   if (e != cudaSuccess) return cfail(RQ_ERR_CUDA, std::string("channel: ") + cudaGetErrorString(e));
   for (int k = 0; k < ch->slots; ++k) __atomic_store_n(&ch->hdr[k].stop, 0u, __ATOMIC_SEQ_CST);
   __atomic_store_n(&ch->ctl->state, kStateRunning, __ATOMIC_SEQ_CST);
-  if (s->tri_kind == kWald)
-    channel_kernel<kWald><<<ch->slots, kChanThreads, smem, ch->stream>>>(A);
-  else
-    channel_kernel<kKS><<<ch->slots, kChanThreads, smem, ch->stream>>>(A);
-  e = cudaGetLastError();
+  void* args[] = {(void*)&A};
+  e = cudaLaunchKernel(f, dim3(ch->slots), dim3(kChanThreads), args, smem, ch->stream);
   if (e != cudaSuccess) {
     __atomic_store_n(&ch->ctl->state, kStateIdle, __ATOMIC_SEQ_CST);
     return cfail(RQ_ERR_CUDA, std::string("channel launch: ") + cudaGetErrorString(e));

@@ -210,6 +210,10 @@ struct DevScene {
   int root_ref;  // >= 0 internal record, < 0 leaf (~first)
   float root_lo[3], root_hi[3];
   int depth;  // maximum number of pending stack entries
+  // four-wide nodes (rq_wide.cu), one per record; NULL: the tree has none
+  const uint32_t* wide;
+  const float4* leaf_box;  // 2 float4 per leaf, at its first triangle: lo xyz hi.x | hi.yz
+  float origin_limit;      // largest |origin| component the wide walk takes
 };
 
 }  // namespace rq

@@ -164,12 +164,8 @@ static int launch(Scene* s, const FrameParams& P, float* rgb, float* t, int32_t*
   B.counters = f->counters;
   B.shadow_rays_ptr = shadow ? shadow : f->shadow;
   B.stats = s->stats;
-  const DevScene S = s->dev();
-  const size_t smem = (size_t)S.depth * 128 * sizeof(int2);
-  const int bps = whitted_blocks_per_sm(s->tri_kind, smem);
-  const int npix = P.xres * P.yres;
-  const int grid = std::max(1, std::min(bps * s->num_sms, (npix + 127) / 128));
-  cudaError_t e = launch_whitted(S, P, B, grid, st, s->stage_events, s->n_stage_events);
+  cudaError_t e = launch_whitted(s->dev(), P, B, s->num_sms, st, s->stage_events,
+                                 s->n_stage_events);
   if (e != cudaSuccess) return set_fail(RQ_ERR_CUDA, std::string("whitted launch: ") +
                                                          cudaGetErrorString(e));
   return RQ_OK;

@@ -31,11 +31,19 @@ struct LaunchPlan {
   int* counter;     // device ray counter (persistent form), zeroed per launch
 };
 
+// Bytes of traversal stack per block: of the binary walk 8 per pending entry
+// not kept in registers (at least one); of the wide walk 4, for at most three
+// refs per two levels, the end mark and one entry past the top.
+inline size_t stack_bytes(int depth, int block, bool wide, int regs = 0) {
+  const int binary = depth - regs > 1 ? depth - regs : 1;
+  return wide ? (size_t)((depth + 1) / 2 * 3 + 2) * block * sizeof(int)
+              : (size_t)binary * block * 2 * sizeof(int);
+}
+
 cudaError_t launch_trace(const DevScene& S, const RayArgs& a, bool anyhit,
                          const LaunchPlan& plan, cudaStream_t st);
 
-int max_blocks_per_sm(int tri_kind, bool anyhit, bool persistent,
-                      int block_threads, size_t smem);
+int max_blocks_per_sm(const DevScene& S, bool anyhit, bool persistent, int block_threads);
 
 // Writes the 48-byte triangle records in leaf order (perm[k] = original
 // triangle id; bit 31 of perm[k] marks the last triangle of a leaf).

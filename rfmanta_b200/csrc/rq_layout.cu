@@ -59,6 +59,7 @@ int Scene::node_layout(int layout, DevScene& S) {
     return RQ_ERR_STATE;
   }
   std::lock_guard<std::mutex> g(mu);
+  S.wide = nullptr;  // its refs are record numbers of the builder's order
   AltLayout& L = alt_layout[layout];
   if (L.nodes && L.generation == generation) {
     S.nodes = L.nodes;

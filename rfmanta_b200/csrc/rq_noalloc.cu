@@ -131,12 +131,8 @@ extern "C" int rq_render_whitted_device_noalloc(rq_scene* scene,
   B.shadow_rays_ptr = d_shadow_rays ? reinterpret_cast<unsigned long long*>(d_shadow_rays)
                                     : reinterpret_cast<unsigned long long*>(base + kOffShadow);
   B.stats = s->stats;
-  const DevScene S = s->dev();
-  const size_t smem = (size_t)S.depth * 128 * sizeof(int2);
-  const int grid = std::max(1, std::min(whitted_blocks_per_sm(s->tri_kind, smem) * s->num_sms,
-                                        (int)((npix + 127) / 128)));
   // launch_whitted clears the work counters and the shadow counter first
-  e = launch_whitted(S, P, B, grid, st, nullptr, 0);
+  e = launch_whitted(s->dev(), P, B, s->num_sms, st, nullptr, 0);
   if (e != cudaSuccess) return na_fail(RQ_ERR_CUDA, std::string("whitted launch: ") + cudaGetErrorString(e));
   return RQ_OK;
 }

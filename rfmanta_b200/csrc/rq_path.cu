@@ -31,6 +31,7 @@
 #include <algorithm>
 
 #include "rq_pathcore.cuh"
+#include "rq_wide.cuh"
 
 namespace rq {
 
@@ -52,18 +53,20 @@ __device__ __forceinline__ int queue_count(const PathBuffers& B, int depth, int 
 // warp's rays finish at different times; results do not depend on the
 // schedule.
 //
-// R = traversal-stack entries kept in registers (0, 1, 2 or 4): the newest
-// pending children stay in registers and only older ones go to this
-// thread's shared-memory column, which holds depth - R entries.
-template <int KIND, bool STATS, int R>
+// Lanes that wait at a leaf, or have ended, before the others stop descending
+// (wide walk): 8 / 12 / 16 / 24 measured 9.45 / 9.25 / 9.20 / 9.23 ms on the
+// 1280x720x16 frame.
+constexpr int kPathVote = 16;
+
+// Walk: the wide walk, or the binary one with its options (statistics,
+// register stack entries) - rq_wide.cuh.
+template <class Walk>
 __global__ void __launch_bounds__(256)
     path_extend_persistent_kernel(DevScene S, PathParams P, PathBuffers B, int depth, int n0,
                                   int refill) {
   extern __shared__ int2 smem_stack[];
-  int2* stk = smem_stack + threadIdx.x;
-  const int stride = blockDim.x;
-  RegStack<R> st;
-  st.init(stk, stride);
+  Walk walk;
+  walk.init(smem_stack);
   const int nq = queue_count(B, depth, n0);
   const int* qin = B.queue[depth & 1];
   int* counter = &B.counters[kFetchBase + depth];
@@ -71,7 +74,6 @@ __global__ void __launch_bounds__(256)
   const unsigned lt_mask = (1u << lane) - 1u;
   int p = -1;  // path slot in flight, -1 = idle
   bool exhausted = false;
-  Counts cnt;
   Ray r;
   Hit h;
   int ref = kDone;
@@ -89,25 +91,21 @@ __global__ void __launch_bounds__(256)
         if (qi < nq) {
           p = depth == 0 ? qi : qin[qi];
           load_extension_ray(B, p, r);
-          start_ray(S, r, h, ref, st.sp);
-          st.nreg = 0;
-          if (STATS) cnt.boxes += 1;
+          walk.start(S, r, false, h, ref);
         } else {
           exhausted = true;
         }
       }
     }
     if (__all_sync(0xffffffffu, exhausted)) break;
-    if (p >= 0) {
-      if (ref != kDone) step_dyn<KIND, R, STATS>(S, r, h, ref, st, false, &cnt);
-      if (ref == kDone) {
-        store_extension(P, B, depth, p, r, h);
-        p = -1;
-      }
+    walk.step(S, r, h, false, p >= 0 && ref != kDone, kPathVote, ref);
+    if (p >= 0 && ref == kDone) {
+      store_extension(P, B, depth, p, r, h);
+      p = -1;
     }
   }
-  if (STATS) {
-    int a = cnt.boxes, b = cnt.tris;
+  if (Walk::STATS) {
+    int a = walk.cnt.boxes, b = walk.cnt.tris;
     for (int o = 16; o > 0; o >>= 1) {
       a += __shfl_xor_sync(0xffffffffu, a, o);
       b += __shfl_xor_sync(0xffffffffu, b, o);
@@ -124,15 +122,13 @@ __global__ void __launch_bounds__(256)
 // steps its shadow ray's any-hit traversal; when the ray is done (or none was
 // needed) it applies shade_finish and the survivors are compacted into the
 // next queue at the warp's common point, one atomic per warp.
-template <int KIND, bool STATS, int R>
+template <class Walk>
 __global__ void __launch_bounds__(256)
     path_shade_persistent_kernel(DevScene S, PathParams P, PathBuffers B, int depth, int n0,
                                  int refill) {
   extern __shared__ int2 smem_stack[];
-  int2* stk = smem_stack + threadIdx.x;
-  const int stride = blockDim.x;
-  RegStack<R> st;
-  st.init(stk, stride);
+  Walk walk;
+  walk.init(smem_stack);
   const int nq = queue_count(B, depth, n0);
   const int* qin = B.queue[depth & 1];
   int* qout = B.queue[(depth + 1) & 1];
@@ -142,7 +138,6 @@ __global__ void __launch_bounds__(256)
   int p = -1;  // path slot in flight, -1 = idle
   bool exhausted = false, alive = false, traced = false;
   int nshadow = 0;
-  Counts cnt;
   float contrib[3];
   Ray sr;
   Hit sh;
@@ -160,13 +155,11 @@ __global__ void __launch_bounds__(256)
         const int qi = base + __popc(m & lt_mask);
         if (qi < nq) {
           p = depth == 0 ? qi : qin[qi];
-          traced = shade_begin<KIND>(S, P, B, depth, p, B.g0 + p, sr, contrib, alive);
+          traced = shade_begin<Walk::KIND>(S, P, B, depth, p, B.g0 + p, sr, contrib, alive);
           ref = kDone;
           if (traced) {
             ++nshadow;
-            start_ray(S, sr, sh, ref, st.sp);
-            st.nreg = 0;
-            if (STATS) cnt.boxes += 1;
+            walk.start(S, sr, true, sh, ref);
           }
         } else {
           exhausted = true;
@@ -175,12 +168,10 @@ __global__ void __launch_bounds__(256)
     }
     if (__all_sync(0xffffffffu, exhausted)) break;
     bool fin = false;
-    if (p >= 0) {
-      if (ref != kDone) step_dyn<KIND, R, STATS>(S, sr, sh, ref, st, true, &cnt);
-      if (ref == kDone) {
-        if (traced && sh.id < 0) shade_finish(B, p, contrib);
-        fin = true;
-      }
+    walk.step(S, sr, sh, true, p >= 0 && ref != kDone, kPathVote, ref);
+    if (p >= 0 && ref == kDone) {
+      if (traced && sh.id < 0) shade_finish(B, p, contrib);
+      fin = true;
     }
     if (B.alive) {
       if (fin) B.alive[p] = alive ? 1 : 0;
@@ -202,8 +193,8 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
   if (lane == 0 && tot) atomicAdd(&B.ray_counts[1], (unsigned long long)tot);
-  if (STATS) {
-    int a = cnt.boxes, b = cnt.tris;
+  if (Walk::STATS) {
+    int a = walk.cnt.boxes, b = walk.cnt.tris;
     for (int o = 16; o > 0; o >>= 1) {
       a += __shfl_xor_sync(0xffffffffu, a, o);
       b += __shfl_xor_sync(0xffffffffu, b, o);
@@ -359,37 +350,45 @@ static int stage_grid(const void* f, int block, int blocks_per_sm, size_t smem) 
   return std::max(1, b * sms);
 }
 
-// Shared-memory stack bytes per block: the column holds the entries that do
-// not fit in the R registers (at least one, so the column is never empty).
-static size_t stack_smem(int depth, int block, int regs) {
-  return (size_t)std::max(1, depth - regs) * block * sizeof(int2);
+// The two stages' kernels: the wide walk where the tree has wide nodes,
+// unless tests are counted or the launch asks for register stack entries,
+// which are the binary walk's.
+struct StageFns {
+  const void *extend, *shade;
+};
+template <class Walk>
+static StageFns stage_fns() {
+  return {(const void*)path_extend_persistent_kernel<Walk>,
+          (const void*)path_shade_persistent_kernel<Walk>};
+}
+template <int KIND, bool STATS>
+static StageFns binary_fns(int regs) {
+  return regs == 4   ? stage_fns<BinaryWalk<KIND, STATS, 4>>()
+         : regs == 2 ? stage_fns<BinaryWalk<KIND, STATS, 2>>()
+         : regs == 1 ? stage_fns<BinaryWalk<KIND, STATS, 1>>()
+                     : stage_fns<BinaryWalk<KIND, STATS, 0>>();
+}
+static StageFns stage_fns(int kind, bool stats, bool wide, int regs) {
+  if (kind == kWald)
+    return wide    ? stage_fns<WideWalk<kWald>>()
+           : stats ? binary_fns<kWald, true>(regs)
+                   : binary_fns<kWald, false>(regs);
+  return wide    ? stage_fns<WideWalk<kKS>>()
+         : stats ? binary_fns<kKS, true>(regs)
+                 : binary_fns<kKS, false>(regs);
 }
 
-template <int KIND, bool STATS>
-static const void* extend_fn(int regs) {
-  return regs == 4 ? (const void*)path_extend_persistent_kernel<KIND, STATS, 4>
-       : regs == 2 ? (const void*)path_extend_persistent_kernel<KIND, STATS, 2>
-       : regs == 1 ? (const void*)path_extend_persistent_kernel<KIND, STATS, 1>
-                   : (const void*)path_extend_persistent_kernel<KIND, STATS, 0>;
-}
-
-template <int KIND, bool STATS>
-static const void* shade_fn(int regs) {
-  return regs == 4 ? (const void*)path_shade_persistent_kernel<KIND, STATS, 4>
-       : regs == 2 ? (const void*)path_shade_persistent_kernel<KIND, STATS, 2>
-       : regs == 1 ? (const void*)path_shade_persistent_kernel<KIND, STATS, 1>
-                   : (const void*)path_shade_persistent_kernel<KIND, STATS, 0>;
-}
-
-template <int KIND, bool STATS>
 static void launch_bounces(const DevScene& S, const PathParams& P, const PathBuffers& B,
                            int n, const PathLaunch& L, cudaStream_t st,
                            const cudaEvent_t* ev, int nev) {
   const int eb = L.block_threads[0], sb = L.block_threads[1];
-  const size_t esm = stack_smem(S.depth, eb, L.reg_stack[0]);
-  const size_t ssm = stack_smem(S.depth, sb, L.reg_stack[1]);
-  const void* ef = extend_fn<KIND, STATS>(L.reg_stack[0]);
-  const void* sf = shade_fn<KIND, STATS>(L.reg_stack[1]);
+  const bool stats = B.stats != nullptr;
+  const bool ew = S.wide && !stats && L.reg_stack[0] == 0;
+  const bool sw = S.wide && !stats && L.reg_stack[1] == 0;
+  const size_t esm = stack_bytes(S.depth, eb, ew, L.reg_stack[0]);
+  const size_t ssm = stack_bytes(S.depth, sb, sw, L.reg_stack[1]);
+  const void* ef = stage_fns(S.tri_kind, stats, ew, L.reg_stack[0]).extend;
+  const void* sf = stage_fns(S.tri_kind, stats, sw, L.reg_stack[1]).shade;
   const int egrid = stage_grid(ef, eb, L.blocks_per_sm[0], esm);
   const int sgrid = stage_grid(sf, sb, L.blocks_per_sm[1], ssm);
   for (int depth = 0; depth < P.max_depth; ++depth) {
@@ -417,31 +416,11 @@ cudaError_t launch_path_chunk(const DevScene& S, const PathParams& P, PathBuffer
   const int ggrid = std::min(grid, (n + 255) / 256);
   path_generate_kernel<<<std::max(ggrid, 1), 256, 0, st>>>(P, B, g0, n);
   if (nev > 0) cudaEventRecord(ev[0], st);
-  const bool stats = B.stats != nullptr;
-  if (S.tri_kind == kWald) {
-    if (stats) launch_bounces<kWald, true>(S, P, B, n, L, st, ev, nev);
-    else launch_bounces<kWald, false>(S, P, B, n, L, st, ev, nev);
-  } else {
-    if (stats) launch_bounces<kKS, true>(S, P, B, n, L, st, ev, nev);
-    else launch_bounces<kKS, false>(S, P, B, n, L, st, ev, nev);
-  }
+  launch_bounces(S, P, B, n, L, st, ev, nev);
   path_resolve_kernel<<<std::max(1, std::min(grid, (n / P.spp + 255) / 256)), 256, 0, st>>>(
       P, B, g0, n, rgb);
   if (nev > 1 + 2 * P.max_depth) cudaEventRecord(ev[1 + 2 * P.max_depth], st);
   return cudaGetLastError();
-}
-
-int path_blocks_per_sm(int tri_kind, size_t smem) {
-  const void* fs[4] = {(const void*)path_shade_persistent_kernel<kWald, false, 0>,
-                       (const void*)path_shade_persistent_kernel<kWald, true, 0>,
-                       (const void*)path_shade_persistent_kernel<kKS, false, 0>,
-                       (const void*)path_shade_persistent_kernel<kKS, true, 0>};
-  if (smem > 48 * 1024)
-    for (const void* f : fs)
-      cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  int b = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fs[tri_kind == kWald ? 0 : 2], 128, smem);
-  return std::max(1, b);
 }
 
 }  // namespace rq

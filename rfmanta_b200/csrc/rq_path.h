@@ -73,7 +73,6 @@ cudaError_t launch_path_chunk(const DevScene& S, const PathParams& P, PathBuffer
                               long long g0, int n, float* rgb, int grid,
                               const PathLaunch& L, cudaStream_t st, const cudaEvent_t* ev,
                               int nev);
-int path_blocks_per_sm(int tri_kind, size_t smem);
 // Builds bounce depth+1's queue (and live count) from B.alive over slots
 // [0, n), in slot order.
 cudaError_t launch_ordered_compaction(const PathBuffers& B, int n, int depth, cudaStream_t st);

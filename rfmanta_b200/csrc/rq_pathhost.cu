@@ -147,8 +147,7 @@ static int path_run(Scene* s, const PathParams& P, long long total, int chunk, f
   DevScene S;
   int lrc = s->node_layout(s->cfg[RQ_PATH_EXTEND].node_layout, S);
   if (lrc != RQ_OK) return lrc;
-  const size_t smem = (size_t)S.depth * 128 * sizeof(int2);
-  const int grid = std::max(1, path_blocks_per_sm(s->tri_kind, smem) * s->num_sms);
+  const int grid = 8 * s->num_sms;  // generate and resolve: eight 256-thread blocks per SM
   PathLaunch L;
   for (int k = 0; k < 2; ++k) {
     const rq_launch_config& c = s->cfg[RQ_PATH_EXTEND + k];

@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -97,6 +98,7 @@ __global__ void refit_root_kernel(const float4* nodes, int root_ref, const float
     out[c] = lo[c];
     out[3 + c] = hi[c];
   }
+  out[6] = 0.f;  // the wide nodes' flag
 }
 
 int Scene::refresh_tree() const {
@@ -157,13 +159,15 @@ int update_tree(Scene* s, int mode) {
                                                  s->d_verts, s->d_idx, s->d_perm);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess && !s->d_root_box) e = cudaMalloc(&s->d_root_box, 6 * sizeof(float));
+  if (e == cudaSuccess && !s->d_root_box) e = cudaMalloc(&s->d_root_box, 7 * sizeof(float));
   if (e == cudaSuccess) {
     refit_root_kernel<<<1, 1>>>(s->d_nodes, s->root_ref, s->d_verts, s->d_idx, s->d_perm,
                                 s->d_root_box);
     e = cudaGetLastError();
   }
-  float root[6];
+  if (e == cudaSuccess)
+    e = s->make_wide(s->n_records, nullptr, reinterpret_cast<int*>(s->d_root_box + 6));
+  float root[7];
   if (e == cudaSuccess)
     e = cudaMemcpy(root, s->d_root_box, sizeof(root), cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) {
@@ -174,6 +178,11 @@ int update_tree(Scene* s, int mode) {
     s->root_lo[c] = root[c];
     s->root_hi[c] = root[3 + c];
   }
+  int wide_bad;
+  std::memcpy(&wide_bad, &root[6], sizeof(int));
+  s->wide_ok = s->n_records > 0 && wide_bad == 0;
+  s->wide_extent = 0.f;
+  for (int k = 0; k < 6; ++k) s->wide_extent = std::max(s->wide_extent, std::fabs(root[k]));
   s->tree_stale = true;
   s->tree_from_dyn = false;
   if (s->dyn) mark_dyn_bounds_stale(s->dyn);

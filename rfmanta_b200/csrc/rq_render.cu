@@ -15,7 +15,7 @@
 #include <algorithm>
 
 #include "rq_render.h"
-#include "rq_traverse.cuh"
+#include "rq_wide.cuh"
 
 namespace rq {
 
@@ -65,8 +65,11 @@ __device__ __forceinline__ void tri_normal(const DevScene& S, int pos,
   }
 }
 
-// Idle lanes a warp gathers before it fetches new pixels.
-constexpr int kWhittedRefill = 8;
+// Idle lanes a warp gathers before it fetches new pixels, and lanes that wait
+// at a leaf, or have ended, before the others stop descending (wide walk).  A
+// 512x512 frame at vote 4 / 8 / 12: 151 / 138 / 136 us, at refill 4 / 8 / 16:
+// 139 / 136 / 134.5 us.
+constexpr int kWhittedRefill = 16, kWhittedVote = 12;
 
 // The Whitted frame in one persistent kernel: each lane takes a pixel, traces
 // its primary ray, and on a hit traces the shadow ray of every point light in
@@ -77,12 +80,13 @@ constexpr int kWhittedRefill = 8;
 // different phases still steps together.  One kernel instead of a primary
 // stage, a compaction and a shade stage: a small frame is bound by the
 // latency of its slowest pixels, and the stages' tails added up.
-template <int KIND, bool STATS>
+template <class Walk>
 __global__ void __launch_bounds__(128)
     whitted_fused_kernel(DevScene S, FrameParams P, FrameBuffers B) {
   extern __shared__ int2 smem_stack[];
-  RegStack<0> st;
-  st.init(smem_stack + threadIdx.x, blockDim.x);
+  constexpr bool STATS = Walk::STATS;
+  Walk walk;
+  walk.init(smem_stack);
   const int npix = P.xres * P.yres;
   int* counter = &B.counters[kCntWork];
   const unsigned lane = threadIdx.x & 31u;
@@ -97,6 +101,11 @@ __global__ void __launch_bounds__(128)
   float ffn[3], total[3];
   int mat = 0, nshadow = 0;
   Counts cp, cs;
+  auto count = [&](Counts& c) {  // moves the walk's counts to c
+    c.boxes += walk.cnt.boxes;
+    c.tris += walk.cnt.tris;
+    walk.cnt = Counts();
+  };
   for (;;) {
     const bool idle = pix < 0 && !exhausted;
     const unsigned m = __ballot_sync(0xffffffffu, idle);
@@ -112,31 +121,17 @@ __global__ void __launch_bounds__(128)
           pix = qi;
           light = -1;
           primary_ray(P, qi % P.xres, qi / P.xres, r);
-          int sp;
-          start_ray(S, r, h, ref, sp);
-          st.sp = 0;
-          if (STATS) cp.boxes += 1;
+          walk.start(S, r, false, h, ref);
+          if (STATS) count(cp);
         } else {
           exhausted = true;
         }
       }
     }
     if (__all_sync(0xffffffffu, exhausted)) break;
-    if (pix < 0) continue;
-    if (ref != kDone) {
-      Counts c;
-      step_dyn<KIND, 0, STATS>(S, r, h, ref, st, light >= 0, &c);
-      if (STATS) {
-        if (light < 0) {
-          cp.boxes += c.boxes;
-          cp.tris += c.tris;
-        } else {
-          cs.boxes += c.boxes;
-          cs.tris += c.tris;
-        }
-      }
-    }
-    if (ref != kDone) continue;
+    walk.step(S, r, h, light >= 0, pix >= 0 && ref != kDone, kWhittedVote, ref);
+    if (STATS) count(light < 0 ? cp : cs);
+    if (pix < 0 || ref != kDone) continue;
     int next;  // first light at or after `next` that sends a shadow ray
     if (light < 0) {
       B.t[pix] = h.t;
@@ -150,7 +145,7 @@ __global__ void __launch_bounds__(128)
         continue;
       }
       float nrm[3];
-      tri_normal<KIND>(S, h.pos, nrm);
+      tri_normal<Walk::KIND>(S, h.pos, nrm);
       const float dn = dot3(nrm, r.d);
 #pragma unroll
       for (int c = 0; c < 3; ++c) ffn[c] = (dn <= 0.f) ? nrm[c] : -nrm[c];
@@ -193,10 +188,8 @@ __global__ void __launch_bounds__(128)
     }
     if (light >= 0) {
       ++nshadow;
-      int sp;
-      start_ray(S, r, h, ref, sp);
-      st.sp = 0;
-      if (STATS) cs.boxes += 1;
+      walk.start(S, r, true, h, ref);
+      if (STATS) count(cs);
       continue;
     }
     const float* kd = P.materials + 3 * (size_t)mat;
@@ -214,42 +207,40 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-cudaError_t launch_whitted(const DevScene& S, const FrameParams& P,
-                           const FrameBuffers& B, int grid, cudaStream_t st,
-                           const cudaEvent_t* ev, int nev) {
+// The frame's kernel: the wide walk where the tree has wide nodes, unless
+// tests are counted.
+static const void* whitted_fn(const DevScene& S, bool stats) {
+  if (S.tri_kind == kWald)
+    return stats     ? (const void*)whitted_fused_kernel<BinaryWalk<kWald, true, 0>>
+           : S.wide ? (const void*)whitted_fused_kernel<WideWalk<kWald>>
+                    : (const void*)whitted_fused_kernel<BinaryWalk<kWald, false, 0>>;
+  return stats     ? (const void*)whitted_fused_kernel<BinaryWalk<kKS, true, 0>>
+         : S.wide ? (const void*)whitted_fused_kernel<WideWalk<kKS>>
+                  : (const void*)whitted_fused_kernel<BinaryWalk<kKS, false, 0>>;
+}
+
+cudaError_t launch_whitted(const DevScene& S, const FrameParams& P, const FrameBuffers& B,
+                           int num_sms, cudaStream_t st, const cudaEvent_t* ev, int nev) {
   const int bs = 128;
-  const size_t smem = (size_t)S.depth * bs * sizeof(int2);
+  const bool stats = B.stats != nullptr;
+  const void* f = whitted_fn(S, stats);
+  const size_t smem = stack_bytes(S.depth, bs, S.wide && !stats);
+  if (smem > 48 * 1024)
+    cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  int b = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, f, bs, smem);
+  const long long npix = (long long)P.xres * P.yres;
+  const int grid = (int)std::max(1LL, std::min((long long)std::max(1, b) * num_sms,
+                                               (npix + bs - 1) / bs));
   cudaError_t e = cudaMemsetAsync(B.counters, 0, kNumCounters * sizeof(int), st);
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(B.shadow_rays_ptr, 0, sizeof(unsigned long long), st);
   if (e != cudaSuccess) return e;
   if (nev > 0) cudaEventRecord(ev[0], st);
-  const bool stats = B.stats != nullptr;
-  if (S.tri_kind == kWald) {
-    if (stats) whitted_fused_kernel<kWald, true><<<grid, bs, smem, st>>>(S, P, B);
-    else whitted_fused_kernel<kWald, false><<<grid, bs, smem, st>>>(S, P, B);
-  } else {
-    if (stats) whitted_fused_kernel<kKS, true><<<grid, bs, smem, st>>>(S, P, B);
-    else whitted_fused_kernel<kKS, false><<<grid, bs, smem, st>>>(S, P, B);
-  }
+  void* args[] = {(void*)&S, (void*)&P, (void*)&B};
+  e = cudaLaunchKernel(f, dim3(grid), dim3(bs), args, smem, st);
   if (nev > 1) cudaEventRecord(ev[1], st);
-  return cudaGetLastError();
-}
-
-int whitted_blocks_per_sm(int tri_kind, size_t smem) {
-  const void* f = tri_kind == kWald ? (const void*)whitted_fused_kernel<kWald, false>
-                                    : (const void*)whitted_fused_kernel<kKS, false>;
-  if (smem > 48 * 1024) {
-    const void* all[4] = {(const void*)whitted_fused_kernel<kWald, false>,
-                          (const void*)whitted_fused_kernel<kWald, true>,
-                          (const void*)whitted_fused_kernel<kKS, false>,
-                          (const void*)whitted_fused_kernel<kKS, true>};
-    for (const void* g : all)
-      cudaFuncSetAttribute(g, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  }
-  int b = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, f, 128, smem);
-  return std::max(1, b);
+  return e;
 }
 
 }  // namespace rq

@@ -80,12 +80,10 @@ __device__ __forceinline__ void primary_ray(const FrameParams& P, int x, int y,
   r.minT = kMaxT;
 }
 
-// The frame's one persistent kernel on `grid` blocks of 128 threads; records
-// ev[0] before it and ev[1] after it when given.
-cudaError_t launch_whitted(const DevScene& S, const FrameParams& P,
-                           const FrameBuffers& B, int grid, cudaStream_t st,
-                           const cudaEvent_t* ev, int nev);
-int whitted_blocks_per_sm(int tri_kind, size_t smem);
+// The frame's one persistent kernel, filling num_sms SMs once; records ev[0]
+// before it and ev[1] after it when given.
+cudaError_t launch_whitted(const DevScene& S, const FrameParams& P, const FrameBuffers& B,
+                           int num_sms, cudaStream_t st, const cudaEvent_t* ev, int nev);
 
 // PinholeCamera::setup (Model/Cameras/PinholeCamera.cc:167-198) on the host.
 void camera_basis(const float* eye, const float* lookat, const float* up,

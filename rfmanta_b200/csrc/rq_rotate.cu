@@ -41,6 +41,7 @@
 
 #include <algorithm>
 #include <cfloat>
+#include <cmath>
 #include <climits>
 #include <cstring>
 #include <string>
@@ -59,6 +60,7 @@ struct UpdState {
   int n_records;
   int depth;
   float root[6];
+  int wide_bad;  // the tree cannot be walked wide (rq_wide.cu)
 };
 
 // Device state of the rotating update: the reference's node array with
@@ -839,6 +841,7 @@ __global__ void init_state_kernel(UpdState* st, int next_free) {
   st->error = 0;
   st->n_records = 0;
   st->depth = 0;
+  st->wide_bad = 0;
 }
 
 // The re-splits' pairs land after next_free; advance it (one thread).
@@ -1001,7 +1004,7 @@ int ensure_record_capacity(Scene* s) {
   if (s->rec_capacity >= need) return RQ_OK;
   float4* nodes = nullptr;
   int32_t* levels = nullptr;
-  DY_CUDA(cudaMalloc(&nodes, (size_t)need * 4 * sizeof(float4)), "record buffer");
+  DY_CUDA(cudaMalloc(&nodes, Scene::record_bytes(need)), "record buffer");
   cudaError_t e = cudaMalloc(&levels, (size_t)need * sizeof(int32_t));
   if (e == cudaSuccess && s->n_records > 0)
     e = cudaMemcpy(nodes, s->d_nodes, (size_t)s->n_records * 4 * sizeof(float4),
@@ -1017,6 +1020,8 @@ int ensure_record_capacity(Scene* s) {
   cudaFree(s->d_nodes);
   cudaFree(s->d_level_recs);
   s->d_nodes = nodes;
+  s->d_wide = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(nodes) +
+                                          Scene::wide_offset(need));
   s->d_level_recs = levels;
   s->rec_capacity = need;
   return RQ_OK;
@@ -1172,6 +1177,7 @@ int rotate_update(Scene* s) {
   DY_CUDA(cudaGetLastError(), "relayout");
   DY_CUDA(launch_tri_setup(s->tri_kind, s->d_verts, s->d_idx, s->d_perm, N, s->d_tris, 0),
           "triangle records");
+  DY_CUDA(s->make_wide(s->rec_capacity, &d.st->n_records, &d.st->wide_bad), "wide nodes");
   UpdState out;
   DY_CUDA(cudaMemcpy(&out, d.st, sizeof(out), cudaMemcpyDeviceToHost), "update state");
   if (out.error != 0) {
@@ -1186,6 +1192,9 @@ int rotate_update(Scene* s) {
   d.layout_host_stale = true;
   s->n_records = out.n_records;
   s->n_leaves = out.n_records + 1;
+  s->wide_ok = out.n_records > 0 && out.wide_bad == 0;
+  s->wide_extent = 0.f;
+  for (float x : out.root) s->wide_extent = std::max(s->wide_extent, std::fabs(x));
   s->root_ref = out.n_records > 0 ? 0 : ~0;
   for (int c = 0; c < 3; ++c) {
     s->root_lo[c] = out.root[c];

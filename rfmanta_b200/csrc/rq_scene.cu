@@ -22,6 +22,7 @@
 #include "rq_device.cuh"
 #include "rq_internal.h"
 #include "rq_scene.h"
+#include "rq_wide.cuh"
 
 namespace rq {
 
@@ -83,11 +84,13 @@ const std::vector<float>* Scene::host_vertices() const {
 }
 
 void Scene::free_tree() {
+  d_wide = nullptr;
+  d_leaf_box = nullptr;
+  wide_ok = false;
   if (d_root_box) cudaFree(d_root_box);
   d_root_box = nullptr;
   if (d_nodes) cudaFree(d_nodes);
   if (d_tris) cudaFree(d_tris);
-  if (d_perm) cudaFree(d_perm);
   if (d_level_recs) cudaFree(d_level_recs);
   d_nodes = nullptr;
   d_tris = nullptr;
@@ -119,6 +122,9 @@ DevScene Scene::dev() const {
     S.root_hi[c] = root_hi[c];
   }
   S.depth = depth > 0 ? depth : 1;
+  S.wide = wide_ok && depth <= kWideMaxDepth ? d_wide : nullptr;
+  S.leaf_box = d_leaf_box;
+  S.origin_limit = kWideOrigin * wide_extent;
   return S;
 }
 
@@ -228,21 +234,27 @@ int Scene::set_tree(const HostTree& t) {
   const std::vector<int32_t>& perm = L.perm;
   // device upload
   free_tree();
-  const size_t rec_bytes = std::max<size_t>(recs.size(), 4) * sizeof(float4);
-  const size_t tri_bytes = std::max<size_t>(perm.size(), 1) * 3 * sizeof(float4);
-  RQ_CUDA(cudaMalloc(&d_nodes, rec_bytes));
-  RQ_CUDA(cudaMalloc(&d_tris, tri_bytes));
+  const int nrec = L.n_records;
+  const int cap = std::max(nrec, 1);
+  RQ_CUDA(cudaMalloc(&d_nodes, record_bytes(cap)));
+  d_wide = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(d_nodes) + wide_offset(cap));
+  // one allocation: triangle records, leaf boxes, leaf order, a flag
+  const size_t np = std::max<size_t>(perm.size(), 1);
+  const size_t box_off = (np * 48 + 255) / 256 * 256, perm_off = box_off + np * 32;
+  RQ_CUDA(cudaMalloc(&d_tris, perm_off + (np + 1) * 4));
+  char* tri_mem = reinterpret_cast<char*>(d_tris);
+  d_leaf_box = reinterpret_cast<float4*>(tri_mem + box_off);
+  d_perm = reinterpret_cast<int32_t*>(tri_mem + perm_off);
+  int* d_bad = d_perm + np;
   if (!recs.empty())
     RQ_CUDA(cudaMemcpy(d_nodes, recs.data(), recs.size() * sizeof(float4),
                        cudaMemcpyHostToDevice));
-  RQ_CUDA(cudaMalloc(&d_perm, std::max<size_t>(perm.size(), 1) * sizeof(int32_t)));
   cudaError_t e = cudaMemcpy(d_perm, perm.data(), perm.size() * sizeof(int32_t),
                              cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
     e = launch_tri_setup(tri_kind, d_verts, d_idx, d_perm, (int)perm.size(),
                          d_tris, 0);
   // records grouped by depth, deepest first (the refit's bottom-up order)
-  const int nrec = L.n_records;
   std::vector<int32_t> by_level(nrec);
   level_offsets.assign(1, 0);
   if (nrec > 0) {
@@ -259,8 +271,15 @@ int Scene::set_tree(const HostTree& t) {
   if (e == cudaSuccess) e = cudaMalloc(&d_level_recs, std::max(nrec, 1) * sizeof(int32_t));
   if (e == cudaSuccess && nrec > 0)
     e = cudaMemcpy(d_level_recs, by_level.data(), nrec * sizeof(int32_t), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  int bad = 1;
+  if (e == cudaSuccess) e = cudaMemset(d_bad, 0, sizeof(int));
+  if (e == cudaSuccess) e = make_wide(nrec, nullptr, d_bad);
+  if (e == cudaSuccess) e = cudaMemcpy(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return cuda_fail(e, "triangle setup");
+  wide_ok = nrec > 0 && bad == 0;
+  wide_extent = 0.f;
+  for (int k = 0; wide_ok && k < 12; ++k)  // the root record's two boxes
+    wide_extent = std::max(wide_extent, std::fabs(reinterpret_cast<const float*>(recs.data())[k]));
   rec_node = L.rec_node;
   rec_depth = L.rec_depth;
   rec_size = L.rec_size;
@@ -383,11 +402,8 @@ LaunchPlan Scene::plan(bool anyhit, int n, int* counter) const {
   p.refill = std::max(1, std::min(32, c.refill_threshold));
   p.counter = counter;
   int bps = c.blocks_per_sm;
-  const size_t smem = (size_t)std::max(depth, 1) * c.block_threads * sizeof(int2);
-  if (bps <= 0)
-    bps = max_blocks_per_sm(tri_kind, anyhit, p.persistent, c.block_threads, smem);
-  else
-    max_blocks_per_sm(tri_kind, anyhit, p.persistent, c.block_threads, smem);
+  const int most = max_blocks_per_sm(dev(), anyhit, p.persistent, c.block_threads);
+  if (bps <= 0) bps = most;
   p.grid = std::max(1, bps * num_sms);
   // never launch more persistent threads than rays
   const int need_blocks = (n + c.block_threads - 1) / c.block_threads;
@@ -415,8 +431,9 @@ int Scene::trace_device(int n, const float* org, const float* dir,
     p.refill = 1;
     p.persistent = false;
     p.counter = nullptr;
-    const size_t smem = (size_t)std::max(depth, 1) * c.block_threads * sizeof(int2);
-    if (smem > 48 * 1024) max_blocks_per_sm(tri_kind, anyhit, false, c.block_threads, smem);
+    const DevScene S = dev();
+    if (stack_bytes(S.depth, c.block_threads, S.wide != nullptr) > 48 * 1024)
+      max_blocks_per_sm(S, anyhit, false, c.block_threads);
   } else {
     p = plan(anyhit, n, counter);
   }

@@ -177,6 +177,20 @@ struct Scene {
     uint64_t generation = ~0ull;
   };
   AltLayout alt_layout[3];
+  // four-wide nodes of the tree (rq_wide.cu), one per record, behind the
+  // records in d_nodes' allocation, and the leaves' boxes, behind the triangle
+  // records in d_tris': made with the tree and after every update.  wide_ok =
+  // the tree can be walked wide; wide_extent = largest coordinate of the root
+  // record's boxes
+  uint32_t* d_wide = nullptr;
+  float4* d_leaf_box = nullptr;
+  bool wide_ok = false;
+  float wide_extent = 0.f;
+  cudaError_t make_wide(int n, const int* n_dev, int* d_bad);
+  // d_nodes' allocation for `cap` records and their wide nodes
+  static size_t record_bytes(int cap) { return wide_offset(cap) + (size_t)cap * 96; }
+  static size_t wide_offset(int cap) { return ((size_t)cap * 64 + 255) / 256 * 256; }
+
   // dev() with the records in `layout` order
   int node_layout(int layout, DevScene& out);
   void free_layouts();

@@ -34,6 +34,7 @@
 #include "rq_pathcore.cuh"
 #include "rq_render.h"
 #include "rq_scene.h"
+#include "rq_wide.cuh"
 
 namespace rq {
 
@@ -96,18 +97,19 @@ __device__ __forceinline__ void stage_scenes(const ServeArgs& A, DevScene* sm) {
 // new path slots (the path tracer's tuned defaults).
 constexpr int kServeExtendRefill = 16;
 constexpr int kServeShadeRefill = 24;
+constexpr int kServeVote = 16;  // wide walk, as the path stages
 
 // Persistent extension stage over the step's live slots: each lane keeps one
 // slot's ray in flight in that slot's request scene; warps refill idle lanes
 // with one atomic on the bounce's work counter (as path_extend_persistent_
 // kernel does for a single frame).
-template <int KIND>
+template <class Walk>
 __global__ void __launch_bounds__(128) serve_extend_kernel(ServeArgs A, PathBuffers B, int depth) {
   extern __shared__ int2 smem_stack[];
   __shared__ DevScene sm_scenes[kMaxServeScenes];
   stage_scenes(A, sm_scenes);
-  int2* stk = smem_stack + threadIdx.x;
-  const int stride = blockDim.x;
+  Walk walk;
+  walk.init(smem_stack);
   const int nq = depth == 0 ? A.n_slots : *(volatile const int*)&B.counters[depth];
   const int* qin = B.queue[depth & 1];
   int* counter = &B.counters[kFetchBase + depth];
@@ -118,7 +120,7 @@ __global__ void __launch_bounds__(128) serve_extend_kernel(ServeArgs A, PathBuff
   bool exhausted = false;
   Ray r;
   Hit h;
-  int ref = kDone, sp = 0;
+  int ref = kDone;
   for (;;) {
     const bool idle = (p < 0) && !exhausted;
     const unsigned m = __ballot_sync(0xffffffffu, idle);
@@ -135,26 +137,20 @@ __global__ void __launch_bounds__(128) serve_extend_kernel(ServeArgs A, PathBuff
           R = &A.reqs[A.slot_req[p]];
           scene = R->scene;
           load_extension_ray(B, p, r);
-          start_ray(sm_scenes[scene], r, h, ref, sp);
+          walk.start(sm_scenes[scene], r, false, h, ref);
         } else {
           exhausted = true;
         }
       }
     }
     if (__all_sync(0xffffffffu, exhausted)) break;
-    if (p >= 0) {
-      if (ref != kDone) {
-        // scene pointers in registers: the stack stores would otherwise make
-        // every node visit read them from shared memory again
-        DevScene S;
-        S.nodes = sm_scenes[scene].nodes;
-        S.tris = sm_scenes[scene].tris;
-        step<KIND, false>(S, r, h, ref, sp, stk, stride);
-      }
-      if (ref == kDone) {
-        store_extension(R->P, B, depth, p, r, h);
-        p = -1;
-      }
+    // scene pointers in registers: the stack stores would otherwise make
+    // every node visit read them from shared memory again
+    const DevScene S = walk_scene<Walk>(sm_scenes[scene]);
+    walk.step(S, r, h, false, p >= 0 && ref != kDone, kServeVote, ref);
+    if (p >= 0 && ref == kDone) {
+      store_extension(R->P, B, depth, p, r, h);
+      p = -1;
     }
   }
 }
@@ -162,13 +158,13 @@ __global__ void __launch_bounds__(128) serve_extend_kernel(ServeArgs A, PathBuff
 // Persistent shade stage: shade_begin, the shadow ray's any-hit steps and
 // shade_finish per lane, survivors compacted into the next queue at the
 // warp's common point.
-template <int KIND>
+template <class Walk>
 __global__ void __launch_bounds__(128) serve_shade_kernel(ServeArgs A, PathBuffers B, int depth) {
   extern __shared__ int2 smem_stack[];
   __shared__ DevScene sm_scenes[kMaxServeScenes];
   stage_scenes(A, sm_scenes);
-  int2* stk = smem_stack + threadIdx.x;
-  const int stride = blockDim.x;
+  Walk walk;
+  walk.init(smem_stack);
   const int nq = depth == 0 ? A.n_slots : *(volatile const int*)&B.counters[depth];
   const int* qin = B.queue[depth & 1];
   int* qout = B.queue[(depth + 1) & 1];
@@ -180,7 +176,7 @@ __global__ void __launch_bounds__(128) serve_shade_kernel(ServeArgs A, PathBuffe
   float contrib[3];
   Ray sr;
   Hit sh;
-  int ref = kDone, sp = 0;
+  int ref = kDone;
   for (;;) {
     const bool idle = (p < 0) && !exhausted;
     const unsigned m = __ballot_sync(0xffffffffu, idle);
@@ -197,12 +193,12 @@ __global__ void __launch_bounds__(128) serve_shade_kernel(ServeArgs A, PathBuffe
           const ServeReq& R = A.reqs[A.slot_req[p]];
           scene = R.scene;
           // a request whose depth is already reached keeps no live paths here
-          traced = shade_begin<KIND>(sm_scenes[scene], R.P, B, depth, p, A.slot_g[p], sr,
+          traced = shade_begin<Walk::KIND>(sm_scenes[scene], R.P, B, depth, p, A.slot_g[p], sr,
                                      contrib, alive);
           ref = kDone;
           if (traced) {
             ++nshadow;
-            start_ray(sm_scenes[scene], sr, sh, ref, sp);
+            walk.start(sm_scenes[scene], sr, true, sh, ref);
           }
         } else {
           exhausted = true;
@@ -211,17 +207,11 @@ __global__ void __launch_bounds__(128) serve_shade_kernel(ServeArgs A, PathBuffe
     }
     if (__all_sync(0xffffffffu, exhausted)) break;
     bool fin = false;
-    if (p >= 0) {
-      if (ref != kDone) {
-        DevScene S;
-        S.nodes = sm_scenes[scene].nodes;
-        S.tris = sm_scenes[scene].tris;
-        step<KIND, true>(S, sr, sh, ref, sp, stk, stride);
-      }
-      if (ref == kDone) {
-        if (traced && sh.id < 0) shade_finish(B, p, contrib);
-        fin = true;
-      }
+    const DevScene S = walk_scene<Walk>(sm_scenes[scene]);
+    walk.step(S, sr, sh, true, p >= 0 && ref != kDone, kServeVote, ref);
+    if (p >= 0 && ref == kDone) {
+      if (traced && sh.id < 0) shade_finish(B, p, contrib);
+      fin = true;
     }
     if (B.alive) {  // survivors are compacted in slot order after the kernel
       if (fin) {
@@ -279,7 +269,7 @@ __global__ void serve_resolve_kernel(ServeArgs A, PathBuffers B) {
   }
 }
 
-template <int KIND>
+template <class Walk>
 static cudaError_t serve_launch_step(const ServeArgs& A, PathBuffers B, int max_depth,
                                      int grid, size_t smem, cudaStream_t st) {
   cudaError_t e = cudaMemsetAsync(B.counters, 0, kPathCounters * sizeof(int), st);
@@ -288,9 +278,9 @@ static cudaError_t serve_launch_step(const ServeArgs& A, PathBuffers B, int max_
   serve_generate_kernel<<<gg, 256, 0, st>>>(A, B);
   for (int depth = 0; depth < max_depth; ++depth) {
     serve_count_kernel<<<1, 32, 0, st>>>(A, B, depth);
-    serve_extend_kernel<KIND><<<grid, 128, smem, st>>>(A, B, depth);
+    serve_extend_kernel<Walk><<<grid, 128, smem, st>>>(A, B, depth);
     cudaMemsetAsync(B.alive, 0, (size_t)A.n_slots, st);
-    serve_shade_kernel<KIND><<<grid, 128, smem, st>>>(A, B, depth);
+    serve_shade_kernel<Walk><<<grid, 128, smem, st>>>(A, B, depth);
     launch_ordered_compaction(B, A.n_slots, depth, st);
   }
   const int rg = std::max(1, std::min(grid, (A.n_pix + 255) / 256));
@@ -298,11 +288,10 @@ static cudaError_t serve_launch_step(const ServeArgs& A, PathBuffers B, int max_
   return cudaGetLastError();
 }
 
-static int serve_blocks_per_sm(int kind, size_t smem) {
-  const void* fs[2] = {kind == kWald ? (const void*)serve_extend_kernel<kWald>
-                                     : (const void*)serve_extend_kernel<kKS>,
-                       kind == kWald ? (const void*)serve_shade_kernel<kWald>
-                                     : (const void*)serve_shade_kernel<kKS>};
+template <class Walk>
+static int serve_blocks_per_sm(size_t smem) {
+  const void* fs[2] = {(const void*)serve_extend_kernel<Walk>,
+                       (const void*)serve_shade_kernel<Walk>};
   int a = 1, b = 1;
   for (const void* f : fs)
     if (smem > 0)  // the static scene table counts against the default 48 KB too
@@ -310,6 +299,23 @@ static int serve_blocks_per_sm(int kind, size_t smem) {
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, fs[0], 128, smem);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fs[1], 128, smem);
   return std::max(1, std::min(a, b));
+}
+
+static int serve_blocks_per_sm(int kind, bool wide, size_t smem) {
+  if (kind == kWald)
+    return wide ? serve_blocks_per_sm<WideWalk<kWald>>(smem)
+                : serve_blocks_per_sm<BinaryWalk<kWald, false, 0>>(smem);
+  return wide ? serve_blocks_per_sm<WideWalk<kKS>>(smem)
+              : serve_blocks_per_sm<BinaryWalk<kKS, false, 0>>(smem);
+}
+
+static cudaError_t serve_launch_step(int kind, bool wide, const ServeArgs& A, const PathBuffers& B,
+                                     int max_depth, int grid, size_t smem, cudaStream_t st) {
+  if (kind == kWald)
+    return wide ? serve_launch_step<WideWalk<kWald>>(A, B, max_depth, grid, smem, st)
+                : serve_launch_step<BinaryWalk<kWald, false, 0>>(A, B, max_depth, grid, smem, st);
+  return wide ? serve_launch_step<WideWalk<kKS>>(A, B, max_depth, grid, smem, st)
+              : serve_launch_step<BinaryWalk<kKS, false, 0>>(A, B, max_depth, grid, smem, st);
 }
 
 }  // namespace rq
@@ -399,6 +405,15 @@ struct rq_server {
   long long steps = 0;
   int grid = 1;
   size_t smem = 0;
+  bool wide = false;  // every scene's tree has wide nodes
+  // walk, stack bytes and grids for the current scenes
+  void size_stacks() {
+    wide = true;
+    for (const rq::DevScene& d : host_scenes) wide = wide && d.wide;
+    smem = rq::stack_bytes(depth, 128, wide);
+    grid = std::max(1, rq::serve_blocks_per_sm(tri_kind, wide, smem) * num_sms);
+    qgrid = std::max(1, rq::batch_blocks_per_sm(tri_kind, 0, wide, 128, smem) * num_sms);
+  }
   // the scenes' descriptors as uploaded and their generations: a scene
   // updated since (refit, rotations, new tree) gets its descriptor copied in
   // again before the next step
@@ -637,11 +652,9 @@ int rq_server_create(rq_scene* const* scenes, int n_scenes, long long path_capac
     if (cudaStreamSynchronize(s->stream) != cudaSuccess)
       return sfail(RQ_ERR_CUDA, "server memory pool");
   }
-  s->smem = (size_t)s->depth * 128 * sizeof(int2);
-  s->grid = std::max(1, serve_blocks_per_sm(s->tri_kind, s->smem) * s->num_sms);
-  s->qgrid = std::max(1, batch_blocks_per_sm(s->tri_kind, 0, 128, s->smem) * s->num_sms);
   s->table.assign(s->max_active, 0);
   s->host_scenes = ds;
+  s->size_stacks();
   for (Scene* sc : s->scenes) s->generations.push_back(sc->generation);
   *out = s.release();
   return RQ_OK;
@@ -753,12 +766,8 @@ int rq_server_step(rq_server* s, int* scheduled_paths) {
                         sizeof(DevScene) * s->host_scenes.size(), cudaMemcpyHostToDevice,
                         s->stream) != cudaSuccess)
       return sfail(RQ_ERR_CUDA, "scene table");
-    if (depth != s->depth) {
-      s->depth = depth;
-      s->smem = (size_t)depth * 128 * sizeof(int2);
-      s->grid = std::max(1, serve_blocks_per_sm(s->tri_kind, s->smem) * s->num_sms);
-      s->qgrid = std::max(1, batch_blocks_per_sm(s->tri_kind, 0, 128, s->smem) * s->num_sms);
-    }
+    s->depth = depth;
+    s->size_stacks();
   }
   // admission in arrival order while the budget allows
   while (!s->pending.empty()) {
@@ -902,7 +911,7 @@ int rq_server_step(rq_server* s, int* scheduled_paths) {
     Q.stats = nullptr;
     e = cudaMemsetAsync(s->d_qcounter, 0, sizeof(int), st);
     const int qg = std::max(1, std::min(s->qgrid, (q_warp_chunks * 32 + 127) / 128));
-    if (e == cudaSuccess) e = launch_batch(s->tri_kind, 0, Q, qg, 128, s->smem, st);
+    if (e == cudaSuccess) e = launch_batch(s->tri_kind, 0, s->wide, Q, qg, 128, s->smem, st);
     s->query_rays += (unsigned long long)qrays;
   }
   // the step's path chunks: one wavefront over all of them
@@ -917,8 +926,7 @@ int rq_server_step(rq_server* s, int* scheduled_paths) {
     A.n_pix = (int)pix;
     A.slot_req = s->slot_req;
     A.slot_g = s->slot_g;
-    e = s->tri_kind == kWald ? serve_launch_step<kWald>(A, s->B, max_depth, s->grid, s->smem, st)
-                             : serve_launch_step<kKS>(A, s->B, max_depth, s->grid, s->smem, st);
+    e = serve_launch_step(s->tri_kind, s->wide, A, s->B, max_depth, s->grid, s->smem, st);
   }
   if (e != cudaSuccess) return sfail(RQ_ERR_CUDA, std::string("serve step: ") + cudaGetErrorString(e));
   for (auto& kv : tidx) {

@@ -19,43 +19,52 @@
 // overflow.
 #include <cuda_runtime.h>
 
-#include "rq_traverse.cuh"
+#include "rq_wide.cuh"
 
 namespace rq {
 
-template <int KIND, bool ANY>
+// Wide walk: lanes of a warp that wait at a leaf, or have ended, before the
+// others stop descending.  Random rays, bound by L1 wavefronts, want the
+// leaves batched (closest hit 209 / 189 / 184 us at 8 / 16 / 24 for 2^20 rays,
+// any hit 507 / 427 / 404 us for 3 M), camera rays, bound by issue slots, the
+// idle lanes short (128 / 137 / 151 us for 777,777).
+constexpr int kClosestVote = 12, kAnyVote = 20;
+
+template <class Walk, bool ANY>
 __global__ void __launch_bounds__(256) trace_kernel(DevScene S, RayArgs a) {
   extern __shared__ int2 smem_stack[];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
-  int2* stk = smem_stack + threadIdx.x;
-  const int stride = blockDim.x;
+  Walk walk;
+  walk.init(smem_stack);
   Ray r;
-  load_ray(a, i, r);
   Hit h;
-  int ref, sp;
-  start_ray(S, r, h, ref, sp);
-  while (ref != kDone) step<KIND, ANY>(S, r, h, ref, sp, stk, stride);
-  store_hit(a, i, h);
+  int ref = kDone;
+  if (i < a.n) {
+    load_ray(a, i, r);
+    walk.start(S, r, ANY, h, ref);
+  }
+  while (__any_sync(0xffffffffu, ref != kDone))
+    walk.step(S, r, h, ANY, ref != kDone, ANY ? kAnyVote : kClosestVote, ref);
+  if (i < a.n) store_hit(a, i, h);
 }
 
-// Persistent form: each lane keeps one ray in flight; after every
-// while-while step the warp counts its idle lanes with a ballot and, once
-// `refill` or more are idle (or none is busy), one lane claims that many ray
-// indices with a single atomicAdd and the idle lanes take them.
-template <int KIND, bool ANY>
+// Persistent form: each lane keeps one ray in flight; after every step the
+// warp counts its idle lanes with a ballot and, once `refill` or more are
+// idle (or none is busy), one lane claims that many ray indices with a single
+// atomicAdd and the idle lanes take them.
+template <class Walk, bool ANY>
 __global__ void __launch_bounds__(256)
     trace_persistent_kernel(DevScene S, RayArgs a, int* counter, int refill) {
   extern __shared__ int2 smem_stack[];
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lt_mask = (1u << lane) - 1u;
-  int2* stk = smem_stack + threadIdx.x;
-  const int stride = blockDim.x;
+  Walk walk;
+  walk.init(smem_stack);
   int idx = -1;  // ray in flight, -1 = idle
   bool exhausted = false;
   Ray r;
   Hit h;
-  int ref = kDone, sp = 0;
+  int ref = kDone;
   for (;;) {
     const bool idle = (idx < 0) && !exhausted;
     const unsigned m = __ballot_sync(0xffffffffu, idle);
@@ -70,63 +79,55 @@ __global__ void __launch_bounds__(256)
         if (mine < a.n) {
           idx = mine;
           load_ray(a, idx, r);
-          start_ray(S, r, h, ref, sp);
+          walk.start(S, r, ANY, h, ref);
         } else {
           exhausted = true;
         }
       }
     }
     if (__all_sync(0xffffffffu, exhausted)) break;
-    if (idx >= 0) {
-      if (ref != kDone) step<KIND, ANY>(S, r, h, ref, sp, stk, stride);
-      if (ref == kDone) {
-        store_hit(a, idx, h);
-        idx = -1;
-      }
+    walk.step(S, r, h, ANY, idx >= 0 && ref != kDone, ANY ? kAnyVote : kClosestVote, ref);
+    if (idx >= 0 && ref == kDone) {
+      store_hit(a, idx, h);
+      idx = -1;
     }
   }
 }
 
-template <int KIND, bool ANY>
-static cudaError_t launch_one(const DevScene& S, const RayArgs& a,
-                              const LaunchPlan& plan, cudaStream_t st) {
-  const size_t smem = (size_t)S.depth * plan.block_threads * sizeof(int2);
-  if (!plan.persistent) {
-    const int grid = (a.n + plan.block_threads - 1) / plan.block_threads;
-    trace_kernel<KIND, ANY><<<grid, plan.block_threads, smem, st>>>(S, a);
-  } else {
-    trace_persistent_kernel<KIND, ANY>
-        <<<plan.grid, plan.block_threads, smem, st>>>(S, a, plan.counter,
-                                                      plan.refill);
-  }
-  return cudaGetLastError();
+// The kernel of a query over this scene: the wide walk where the tree has
+// wide nodes.
+template <class Walk>
+static const void* trace_fn(bool any, bool persistent) {
+  if (persistent)
+    return any ? (const void*)trace_persistent_kernel<Walk, true>
+               : (const void*)trace_persistent_kernel<Walk, false>;
+  return any ? (const void*)trace_kernel<Walk, true> : (const void*)trace_kernel<Walk, false>;
+}
+
+static const void* trace_fn(const DevScene& S, bool any, bool persistent) {
+  if (S.tri_kind == kWald)
+    return S.wide ? trace_fn<WideWalk<kWald>>(any, persistent)
+                  : trace_fn<BinaryWalk<kWald, false, 0>>(any, persistent);
+  return S.wide ? trace_fn<WideWalk<kKS>>(any, persistent)
+                : trace_fn<BinaryWalk<kKS, false, 0>>(any, persistent);
 }
 
 cudaError_t launch_trace(const DevScene& S, const RayArgs& a, bool anyhit,
                          const LaunchPlan& plan, cudaStream_t st) {
   if (a.n <= 0) return cudaSuccess;
-  if (S.tri_kind == kWald)
-    return anyhit ? launch_one<kWald, true>(S, a, plan, st)
-                  : launch_one<kWald, false>(S, a, plan, st);
-  return anyhit ? launch_one<kKS, true>(S, a, plan, st)
-                : launch_one<kKS, false>(S, a, plan, st);
+  const void* f = trace_fn(S, anyhit, plan.persistent);
+  const size_t smem = stack_bytes(S.depth, plan.block_threads, S.wide != nullptr);
+  const int grid = plan.persistent ? plan.grid
+                                   : (a.n + plan.block_threads - 1) / plan.block_threads;
+  void* args[] = {(void*)&S, (void*)&a, (void*)&plan.counter, (void*)&plan.refill};
+  return cudaLaunchKernel(f, dim3(grid), dim3(plan.block_threads), args, smem, st);
 }
 
-// Occupancy-derived resident blocks per SM for the persistent form.
-int max_blocks_per_sm(int tri_kind, bool anyhit, bool persistent,
-                      int block_threads, size_t smem) {
+// Occupancy-derived resident blocks per SM.
+int max_blocks_per_sm(const DevScene& S, bool anyhit, bool persistent, int block_threads) {
   int nb = 0;
-  const void* f = nullptr;
-  if (tri_kind == kWald)
-    f = persistent ? (anyhit ? (const void*)trace_persistent_kernel<kWald, true>
-                             : (const void*)trace_persistent_kernel<kWald, false>)
-                   : (anyhit ? (const void*)trace_kernel<kWald, true>
-                             : (const void*)trace_kernel<kWald, false>);
-  else
-    f = persistent ? (anyhit ? (const void*)trace_persistent_kernel<kKS, true>
-                             : (const void*)trace_persistent_kernel<kKS, false>)
-                   : (anyhit ? (const void*)trace_kernel<kKS, true>
-                             : (const void*)trace_kernel<kKS, false>);
+  const void* f = trace_fn(S, anyhit, persistent);
+  const size_t smem = stack_bytes(S.depth, block_threads, S.wide != nullptr);
   if (smem > 48 * 1024)
     cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)smem);

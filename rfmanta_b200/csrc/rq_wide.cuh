@@ -1,0 +1,353 @@
+// Four-wide traversal of the binary tree, with the binary walk's results.
+//
+// A wide node holds the (up to four) grandchildren of a node record in
+// 96 bytes: their boxes as 16-bit centre and half extent in the node's own
+// cube, padded outwards, their refs, and the three split axes (layout in
+// rq_wide.cu).  One visit replaces two to three dependent record visits and
+// tests four boxes with packed 16-bit arithmetic.
+//
+// Why the results are the binary walk's, bit for bit:
+//   * the four children are taken in the binary walk's order, which each of
+//     the three folded records fixes by its axis and the ray's direction
+//     signs (closest hit) or its isLeftCheaper flag (any hit);
+//   * a 16-bit box only decides what is skipped, and it contains the exact
+//     box by more than all rounding errors (bound below), so no leaf that the
+//     binary walk tests is skipped;
+//   * a leaf's exact box test (box_test, the current minT) is made before a
+//     hit in it is accepted.  Node boxes are nested (checked when the wide
+//     nodes are made) and rounding is monotonic, so every record above a leaf
+//     whose exact box is hit was hit too, with a minT at least as large: the
+//     leaf's own test stands for the whole chain.
+//
+// Error bound.  In units of the node's cube, with u = 2^-11 (half rounding),
+// the reference point is the ray's closest point to the cube's centre, within
+// 0.87 of it when the ray meets the cube, so a plane lies within 1.37 of it.
+// The plane's time carries errors of 0.87 u (offset) + 0.5 u (slope) + 1.37 u
+// (centre) + 0.5 u (extent) + 1.37 u (sum) < 2.3e-3, the 32-bit origin and
+// slope and the exact test's own rounding 7 * 2^-24 * |origin| with |origin|
+// <= 2048 cube sizes (kWideOrigin bounds the ray, kWideMinCube the cube)
+// < 0.9e-3; the padding is kWidePad = 3.9e-3.  Times against minT: 2^-8 slack.
+//
+// What it is for: the binary walk is bound by issue slots (52-57% issued, 10-15
+// of 32 lanes) and by the dependent record loads (13 to 31 visits a ray), and on
+// random rays by L1 wavefronts (79% busy).  The wide walk makes 1.7 times fewer
+// visits, reads a node in three loads for a record's four, and votes: a warp
+// stops descending once enough lanes wait at leaves, so leaves are tested by
+// more lanes together.  Measured against the binary walk: 777,777 camera rays
+// 246 -> 144 us, 2^20 random closest hits 234 -> 195 us, 3 M random occlusion
+// rays 578 -> 415 us, the 1280x720x16 path frame 11.38 -> 9.19 ms, the 512x512
+// Whitted frame 224 -> 138 us.  Eight-wide nodes would save a third more
+// visits but cost as many instructions a ray (more order to keep) and more L1
+// wavefronts; 8-bit boxes halve the bytes but need twice the padding.
+//
+// Rays outside these bounds (an infinite inverse direction, a slope above
+// kWideSlope, an origin farther than kWideOrigin scene sizes) take the exact
+// binary walk with a stack in local memory (wide_trace_exact).
+#pragma once
+
+#include <cuda_fp16.h>
+
+#include "rq_traverse.cuh"
+
+namespace rq {
+
+constexpr float kWidePad = 1.f / 256;
+constexpr float kWideSlope = 16384.f;   // largest |d|max / |d_k|
+constexpr float kWideOrigin = 16.f;     // largest |origin| over the scene's largest |coordinate|
+// smallest cube over the scene's largest |coordinate|: |origin - centre| stays
+// below 2048 cubes
+constexpr float kWideMinCube = (kWideOrigin + 1.f) / 2048.f;
+constexpr int kWideMaxDepth = 64;       // binary depth the local-memory stack takes
+
+// What a wide visit needs of a ray beside the Ray itself.
+struct WideRay {
+  float A[3];         // |d|max / d_k
+  float w[3];         // -(d_k / |d|max) / sum (d_k / |d|max)^2
+  __half2 a2[3];      // A, both halves
+  __half2 p2[3];      // |A|, both halves
+  float dm;           // |d|max
+  unsigned side;      // bit k: d_k > 0 (closest hit); 8: any hit; for each folded record
+};
+
+// Prepares a ray; false when it must take the exact walk.
+__device__ __forceinline__ bool wide_setup(const DevScene& S, const Ray& r, bool any,
+                                           WideRay& w) {
+  const float ax = fabsf(r.d[0]), ay = fabsf(r.d[1]), az = fabsf(r.d[2]);
+  w.dm = fmaxf(fmaxf(ax, ay), az);
+  bool ok = w.dm > 1e-15f && w.dm < 1e15f && !(r.minT != r.minT);
+  const float rd = __fdividef(1.f, w.dm);
+  float g[3], sum = 0.f;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    w.A[c] = w.dm * r.inv[c];
+    ok = ok && fabsf(w.A[c]) <= kWideSlope && fabsf(r.o[c]) <= S.origin_limit;
+    g[c] = r.d[c] * rd;
+    sum = __fmaf_rn(g[c], g[c], sum);
+    w.a2[c] = __float2half2_rn(w.A[c]);
+    w.p2[c] = __habs2(w.a2[c]);
+  }
+  const float k = __fdividef(-1.f, sum);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) w.w[c] = g[c] * k;
+  w.side = 0x111u * (any ? 8u
+                         : (r.d[0] > 0.f ? 1u : 0u) | (r.d[1] > 0.f ? 2u : 0u) |
+                               (r.d[2] > 0.f ? 4u : 0u));
+  return ok;
+}
+
+struct Words8 {
+  uint32_t x[8];
+};
+__device__ __forceinline__ Words8 load_words8(const void* p) {
+  Words8 r;
+  asm("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+      : "=r"(r.x[0]), "=r"(r.x[1]), "=r"(r.x[2]), "=r"(r.x[3]), "=r"(r.x[4]), "=r"(r.x[5]),
+        "=r"(r.x[6]), "=r"(r.x[7])
+      : "l"(p));
+  return r;
+}
+__device__ __forceinline__ __half2 as_half2(uint32_t x) {
+  __half2 h;
+  memcpy(&h, &x, 4);
+  return h;
+}
+__device__ __forceinline__ uint32_t as_word(__half2 h) {
+  uint32_t x;
+  memcpy(&x, &h, 4);
+  return x;
+}
+
+// refs a, b where the packed comparison near <= far holds, else kDone
+__device__ __forceinline__ void keep_hit(__half2 near, __half2 far, int& a, int& b) {
+  asm("{\n\t.reg .pred p, q;\n\tsetp.le.f16x2 p|q, %2, %3;\n\t"
+      "selp.b32 %0, %0, 0x7fffffff, p;\n\tselp.b32 %1, %1, 0x7fffffff, q;\n\t}"
+      : "+r"(a), "+r"(b)
+      : "r"(as_word(near)), "r"(as_word(far)));
+}
+
+// A lane's stack of refs in shared memory: `top` is the shared-memory address
+// of the next entry, entries `step` bytes apart (one column per thread).
+struct WideStack {
+  uint32_t base, top, step;
+  __device__ __forceinline__ void init(int* column, int stride) {
+    base = (uint32_t)__cvta_generic_to_shared(column);
+    step = (uint32_t)stride * 4u;
+    top = base;
+  }
+  // empties it down to its end mark, which the last pop returns
+  __device__ __forceinline__ void reset() {
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(base), "r"(kDone) : "memory");
+    top = base + step;
+  }
+  __device__ __forceinline__ int pop() {
+    int r;
+    top -= step;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r) : "r"(top) : "memory");
+    return r;
+  }
+  // stores x beyond the top and keeps it there unless it is kDone
+  __device__ __forceinline__ void push_hit(int x) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tst.shared.u32 [%0], %1;\n\t"
+        "setp.ne.s32 p, %1, 0x7fffffff;\n\t@p add.u32 %0, %0, %2;\n\t}"
+        : "+r"(top)
+        : "r"(x), "r"(step)
+        : "memory");
+  }
+};
+
+// One wide node: the children hit are pushed, last to visit first, and the
+// top of the stack (a child, or an older ref when none was hit) is popped.
+__device__ __forceinline__ void wide_visit(const DevScene& S, const Ray& r, const WideRay& w,
+                                           int& ref, WideStack& st) {
+  const char* p = reinterpret_cast<const char*>(S.wide) + 96 * (size_t)ref;
+  const Words8 u0 = load_words8(p), u1 = load_words8(p + 32), u2 = load_words8(p + 64);
+  const float gs = __uint_as_float(u0.x[3]);
+  float o[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) o[c] = __fmaf_rn(r.o[c], gs, -__uint_as_float(u0.x[c]));
+  // time of the point closest to the cube's centre, in cube units
+  const float tm = __fmaf_rn(o[0], w.w[0], __fmaf_rn(o[1], w.w[1], o[2] * w.w[2]));
+  constexpr float slack = 1.f / 256;
+  const __half2 lo = __float2half2_rn(-tm - slack);
+  const __half2 hi = __float2half2_rn(__fmaf_rn(r.minT * w.dm, gs, slack - tm));
+  __half2 near01 = lo, near23 = lo, far01 = hi, far23 = hi;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const __half2 b = __float2half2_rn(__fmaf_rn(-o[c], w.A[c], -tm));
+    const __half2 c01 = as_half2(c == 0 ? u1.x[0] : c == 1 ? u1.x[2] : u1.x[4]);
+    const __half2 c23 = as_half2(c == 0 ? u1.x[1] : c == 1 ? u1.x[3] : u1.x[5]);
+    const __half2 h01 = as_half2(c == 0 ? u1.x[6] : c == 1 ? u2.x[0] : u2.x[2]);
+    const __half2 h23 = as_half2(c == 0 ? u1.x[7] : c == 1 ? u2.x[1] : u2.x[3]);
+    const __half2 t01 = __hfma2(c01, w.a2[c], b), t23 = __hfma2(c23, w.a2[c], b);
+    near01 = __hmax2(near01, __hfma2(__hneg2(h01), w.p2[c], t01));
+    near23 = __hmax2(near23, __hfma2(__hneg2(h23), w.p2[c], t23));
+    far01 = __hmin2(far01, __hfma2(h01, w.p2[c], t01));
+    far23 = __hmin2(far23, __hfma2(h23, w.p2[c], t23));
+  }
+  int r0 = (int)u0.x[4], r1 = (int)u0.x[5], r2 = (int)u0.x[6], r3 = (int)u0.x[7];
+  keep_hit(near01, far01, r0, r1);
+  keep_hit(near23, far23, r2, r3);
+  // the binary order: within each side, then the sides
+  const unsigned m = u2.x[4] & w.side;
+  const bool f0 = (m & 0xfu) != 0u, f1 = (m & 0xf0u) != 0u, f2 = (m & 0xf00u) != 0u;
+  const int a0 = f1 ? r0 : r1, a1 = f1 ? r1 : r0;
+  const int b0 = f2 ? r2 : r3, b1 = f2 ? r3 : r2;
+  st.push_hit(f0 ? b1 : a1);
+  st.push_hit(f0 ? b0 : a0);
+  st.push_hit(f0 ? a1 : b1);
+  st.push_hit(f0 ? a0 : b0);
+  ref = st.pop();
+}
+
+// A leaf's triangles; the first accepted hit is preceded by the leaf's exact
+// box test with the minT the leaf was entered with.  Pops the next ref.
+template <int KIND>
+__device__ __forceinline__ void wide_leaf(const DevScene& S, Ray& r, Hit& h, bool any, int& ref,
+                                          WideStack& st) {
+  const int first = ~ref;
+  const float4* p = S.tris + 3 * (size_t)first;
+  bool in_box = false;
+  for (;;) {
+    bool last;
+    const float t_in = r.minT;
+    Hit n;
+    const bool hit = tri_test<KIND>(r, p, n, last);
+    if (hit) {
+      if (!in_box) {
+        const Words8 b = load_words8(S.leaf_box + 2 * (size_t)first);
+        const float t_hit = r.minT;
+        r.minT = t_in;
+        float te;
+        in_box = box_test(r, __uint_as_float(b.x[0]), __uint_as_float(b.x[1]),
+                          __uint_as_float(b.x[2]), __uint_as_float(b.x[3]),
+                          __uint_as_float(b.x[4]), __uint_as_float(b.x[5]), te);
+        if (!in_box) break;
+        r.minT = t_hit;
+      }
+      h = n;
+      h.pos = (int)((p - S.tris) / 3);
+      if (any) {
+        ref = kDone;
+        return;
+      }
+    }
+    if (last) break;
+    p += 3;
+  }
+  ref = st.pop();
+}
+
+// The exact binary walk to its end, for rays wide_setup refuses.  Arguments
+// and result by value: the callers' ray and hit stay in registers.
+template <int KIND, bool ANY>
+__device__ __noinline__ Hit wide_trace_exact(const float4* nodes, const float4* tris, int ref,
+                                             Ray r) {
+  DevScene S;
+  S.nodes = nodes;
+  S.tris = tris;
+  Hit h;
+  h.id = -1;
+  h.pos = -1;
+  h.t = r.minT;
+  h.u = h.v = 0.f;
+  int2 stk[kWideMaxDepth];
+  int sp = 0;
+  while (ref != kDone) step<KIND, ANY>(S, r, h, ref, sp, stk, 1);
+  return h;
+}
+
+// A ray's start: root box, and the whole exact walk where it must be taken.
+// ref = kDone when the ray is finished.  The column's first entry is the end
+// mark that the last pop returns.
+template <int KIND>
+__device__ __forceinline__ void wide_start(const DevScene& S, Ray& r, bool any, WideRay& w,
+                                           Hit& h, int& ref, WideStack& st) {
+  const bool ok = wide_setup(S, r, any, w);
+  int sp;
+  start_ray(S, r, h, ref, sp);
+  if (!ok && ref != kDone) {
+    h = any ? wide_trace_exact<KIND, true>(S.nodes, S.tris, ref, r)
+            : wide_trace_exact<KIND, false>(S.nodes, S.tris, ref, r);
+    ref = kDone;
+  }
+  st.reset();
+}
+
+// Node visits of a whole warp until `vote` of its live lanes wait at a leaf
+// or at their end, then the waiting leaves.  Called by all 32 lanes.
+template <int KIND>
+__device__ __forceinline__ void wide_step(const DevScene& S, Ray& r, const WideRay& w, Hit& h,
+                                          bool any, bool live, int vote, int& ref,
+                                          WideStack& st) {
+  const int stop = max(0, __popc(__ballot_sync(0xffffffffu, live)) - vote);
+  for (;;) {
+    const bool inner = live && (unsigned)ref < (unsigned)kDone;
+    if (__popc(__ballot_sync(0xffffffffu, inner)) <= stop) break;
+    if (inner) wide_visit(S, r, w, ref, st);
+  }
+  if (live && ref < 0) wide_leaf<KIND>(S, r, h, any, ref, st);
+}
+
+// The two walks behind one interface, for kernels whose warps keep one ray per
+// lane in flight: init once, start per ray (ref = kDone when it is finished
+// already), step by the whole warp with `live` where ref != kDone.
+
+// Binary walk over the node records, R stack entries in registers; a step of
+// a lane runs to its next leaf and through it.
+template <int KIND_, bool STATS_, int R>
+struct BinaryWalk {
+  static constexpr int KIND = KIND_;
+  static constexpr bool STATS = STATS_, WIDE = false;
+  RegStack<R> st;
+  Counts cnt;
+  __device__ __forceinline__ void init(void* smem) {
+    st.init(static_cast<int2*>(smem) + threadIdx.x, blockDim.x);
+  }
+  __device__ __forceinline__ void start(const DevScene& S, Ray& r, bool any, Hit& h, int& ref) {
+    start_ray(S, r, h, ref, st.sp);
+    st.nreg = 0;
+    if (STATS) cnt.boxes += 1;
+  }
+  __device__ __forceinline__ void step(const DevScene& S, Ray& r, Hit& h, bool any, bool live,
+                                       int vote, int& ref) {
+    if (live) step_dyn<KIND, R, STATS>(S, r, h, ref, st, any, &cnt);
+  }
+};
+
+// Wide walk; needs S.wide.
+template <int KIND_>
+struct WideWalk {
+  static constexpr int KIND = KIND_;
+  static constexpr bool STATS = false, WIDE = true;
+  WideStack st;
+  WideRay w;
+  Counts cnt;  // stays zero
+  __device__ __forceinline__ void init(void* smem) {
+    st.init(static_cast<int*>(smem) + threadIdx.x, blockDim.x);
+  }
+  __device__ __forceinline__ void start(const DevScene& S, Ray& r, bool any, Hit& h, int& ref) {
+    wide_start<KIND>(S, r, any, w, h, ref, st);
+  }
+  __device__ __forceinline__ void step(const DevScene& S, Ray& r, Hit& h, bool any, bool live,
+                                       int vote, int& ref) {
+    wide_step<KIND>(S, r, w, h, any, live, vote, ref, st);
+  }
+};
+
+// The pointers a walk's steps follow, copied from a scene table in shared
+// memory.
+template <class Walk>
+__device__ __forceinline__ DevScene walk_scene(const DevScene& s) {
+  DevScene S;
+  S.tris = s.tris;
+  if (Walk::WIDE) {
+    S.wide = s.wide;
+    S.leaf_box = s.leaf_box;
+  } else {
+    S.nodes = s.nodes;
+  }
+  return S;
+}
+
+}  // namespace rq
