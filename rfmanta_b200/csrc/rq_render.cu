@@ -82,7 +82,8 @@ constexpr int kWhittedRefill = 16, kWhittedVote = 12;
 // latency of its slowest pixels, and the stages' tails added up.
 template <class Walk>
 __global__ void __launch_bounds__(128)
-    whitted_fused_kernel(DevScene S, FrameParams P, FrameBuffers B) {
+    whitted_fused_kernel(const __grid_constant__ DevScene S,
+                         const __grid_constant__ FrameParams P, FrameBuffers B) {
   extern __shared__ int2 smem_stack[];
   constexpr bool STATS = Walk::STATS;
   Walk walk;

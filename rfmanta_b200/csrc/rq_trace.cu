@@ -31,7 +31,8 @@ namespace rq {
 constexpr int kClosestVote = 12, kAnyVote = 20;
 
 template <class Walk, bool ANY>
-__global__ void __launch_bounds__(256) trace_kernel(DevScene S, RayArgs a) {
+__global__ void __launch_bounds__(256) trace_kernel(const __grid_constant__ DevScene S,
+                                                    RayArgs a) {
   extern __shared__ int2 smem_stack[];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   Walk walk;
@@ -54,7 +55,8 @@ __global__ void __launch_bounds__(256) trace_kernel(DevScene S, RayArgs a) {
 // atomicAdd and the idle lanes take them.
 template <class Walk, bool ANY>
 __global__ void __launch_bounds__(256)
-    trace_persistent_kernel(DevScene S, RayArgs a, int* counter, int refill) {
+    trace_persistent_kernel(const __grid_constant__ DevScene S, RayArgs a, int* counter,
+                            int refill) {
   extern __shared__ int2 smem_stack[];
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lt_mask = (1u << lane) - 1u;

@@ -19,14 +19,16 @@
 //     whose exact box is hit was hit too, with a minT at least as large: the
 //     leaf's own test stands for the whole chain.
 //
-// Error bound.  In units of the node's cube, with u = 2^-11 (half rounding),
-// the reference point is the ray's closest point to the cube's centre, within
-// 0.87 of it when the ray meets the cube, so a plane lies within 1.37 of it.
-// The plane's time carries errors of 0.87 u (offset) + 0.5 u (slope) + 1.37 u
-// (centre) + 0.5 u (extent) + 1.37 u (sum) < 2.3e-3, the 32-bit origin and
-// slope and the exact test's own rounding 7 * 2^-24 * |origin| with |origin|
-// <= 2048 cube sizes (kWideOrigin bounds the ray, kWideMinCube the cube)
-// < 0.9e-3; the padding is kWidePad = 3.9e-3.  Times against minT: 2^-8 slack.
+// Error bound.  In units of the node's cube (half size at most 0.57 with its
+// padding), with u = 2^-11 (half rounding), the reference point is the ray's
+// closest point to the cube's centre, within 0.98 of it when the ray meets the
+// cube, so a plane lies within 1.5 of it.  A plane's time carries errors of
+// 0.98 u (offset) + 0.5 u (slope) + 1.5 u (centre) + 0.53 u (extent) + 1.5 u
+// (sum) < 2.5e-3 = kWidePad, and those of the 32-bit origin and slope and of
+// the exact test's own rounding, 7 * 2^-24 of the distance to the origin, which
+// is below (kWideOrigin + 1) scene sizes: kWidePad32 of that is added, in the
+// scene's units (and bounds the smallest cube).  Times against minT carry a
+// slack of 2^-8 cubes and 2^-22 of the distance.
 //
 // What it is for: the binary walk is bound by issue slots (52-57% issued, 10-15
 // of 32 lanes) and by the dependent record loads (13 to 31 visits a ray), and on
@@ -51,12 +53,12 @@
 
 namespace rq {
 
-constexpr float kWidePad = 1.f / 256;
+constexpr float kWidePad = 2.5e-3f;
+constexpr float kWidePad32 = 4.8e-7f;   // 8 * 2^-24
 constexpr float kWideSlope = 16384.f;   // largest |d|max / |d_k|
-constexpr float kWideOrigin = 16.f;     // largest |origin| over the scene's largest |coordinate|
-// smallest cube over the scene's largest |coordinate|: |origin - centre| stays
-// below 2048 cubes
-constexpr float kWideMinCube = (kWideOrigin + 1.f) / 2048.f;
+constexpr float kWideOrigin = 64.f;     // largest |origin| over the scene's largest |coordinate|
+// cubes are at least 16 times the 32-bit padding
+constexpr float kWideMinCube = 16.f * kWidePad32 * (kWideOrigin + 1.f);
 constexpr int kWideMaxDepth = 64;       // binary depth the local-memory stack takes
 
 // What a wide visit needs of a ray beside the Ray itself.
@@ -65,6 +67,7 @@ struct WideRay {
   float w[3];         // -(d_k / |d|max) / sum (d_k / |d|max)^2
   __half2 a2[3];      // A, both halves
   __half2 p2[3];      // |A|, both halves
+  __half2 n2[3];      // -|A|
   float dm;           // |d|max
   unsigned side;      // bit k: d_k > 0 (closest hit); 8: any hit; for each folded record
 };
@@ -85,6 +88,7 @@ __device__ __forceinline__ bool wide_setup(const DevScene& S, const Ray& r, bool
     sum = __fmaf_rn(g[c], g[c], sum);
     w.a2[c] = __float2half2_rn(w.A[c]);
     w.p2[c] = __habs2(w.a2[c]);
+    w.n2[c] = __hneg2(w.p2[c]);
   }
   const float k = __fdividef(-1.f, sum);
 #pragma unroll
@@ -94,6 +98,11 @@ __device__ __forceinline__ bool wide_setup(const DevScene& S, const Ray& r, bool
                                (r.d[2] > 0.f ? 4u : 0u));
   return ok;
 }
+
+// Node visits between two votes: 2 against 1 saves the loop's overhead (camera
+// rays 131.6 -> 128.3 us, random any hit 408 -> 401 us, 24 batches 629 -> 614
+// us); at 3 the path stages lose 5% to idle lanes.
+constexpr int kWideVisits = 2;
 
 struct Words8 {
   uint32_t x[8];
@@ -168,7 +177,7 @@ __device__ __forceinline__ void wide_visit(const DevScene& S, const Ray& r, cons
   for (int c = 0; c < 3; ++c) o[c] = __fmaf_rn(r.o[c], gs, -__uint_as_float(u0.x[c]));
   // time of the point closest to the cube's centre, in cube units
   const float tm = __fmaf_rn(o[0], w.w[0], __fmaf_rn(o[1], w.w[1], o[2] * w.w[2]));
-  constexpr float slack = 1.f / 256;
+  const float slack = __fmaf_rn(fabsf(tm), 2.4e-7f, 1.f / 256);
   const __half2 lo = __float2half2_rn(-tm - slack);
   const __half2 hi = __float2half2_rn(__fmaf_rn(r.minT * w.dm, gs, slack - tm));
   __half2 near01 = lo, near23 = lo, far01 = hi, far23 = hi;
@@ -180,8 +189,8 @@ __device__ __forceinline__ void wide_visit(const DevScene& S, const Ray& r, cons
     const __half2 h01 = as_half2(c == 0 ? u1.x[6] : c == 1 ? u2.x[0] : u2.x[2]);
     const __half2 h23 = as_half2(c == 0 ? u1.x[7] : c == 1 ? u2.x[1] : u2.x[3]);
     const __half2 t01 = __hfma2(c01, w.a2[c], b), t23 = __hfma2(c23, w.a2[c], b);
-    near01 = __hmax2(near01, __hfma2(__hneg2(h01), w.p2[c], t01));
-    near23 = __hmax2(near23, __hfma2(__hneg2(h23), w.p2[c], t23));
+    near01 = __hmax2(near01, __hfma2(h01, w.n2[c], t01));
+    near23 = __hmax2(near23, __hfma2(h23, w.n2[c], t23));
     far01 = __hmin2(far01, __hfma2(h01, w.p2[c], t01));
     far23 = __hmin2(far23, __hfma2(h23, w.p2[c], t23));
   }
@@ -281,10 +290,10 @@ __device__ __forceinline__ void wide_step(const DevScene& S, Ray& r, const WideR
                                           bool any, bool live, int vote, int& ref,
                                           WideStack& st) {
   const int stop = max(0, __popc(__ballot_sync(0xffffffffu, live)) - vote);
-  for (;;) {
-    const bool inner = live && (unsigned)ref < (unsigned)kDone;
-    if (__popc(__ballot_sync(0xffffffffu, inner)) <= stop) break;
-    if (inner) wide_visit(S, r, w, ref, st);
+  while (__popc(__ballot_sync(0xffffffffu, live && (unsigned)ref < (unsigned)kDone)) > stop) {
+#pragma unroll
+    for (int k = 0; k < kWideVisits; ++k)
+      if (live && (unsigned)ref < (unsigned)kDone) wide_visit(S, r, w, ref, st);
   }
   if (live && ref < 0) wide_leaf<KIND>(S, r, h, any, ref, st);
 }
