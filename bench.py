@@ -1195,11 +1195,10 @@ class AnimatedFrame(SmallFrame):
                            for v in self.poses]
         self.sc.mesh.vertices = self.poses[0]
         bvh.update()
-        # kernels per step: 1 for the frame; the update's state reset, object
-        # boxes, leaf boxes, re-splits, 2 scan kernels, relocation, next-free
-        # advance, rotations, parents, 1 + 9 pointer-jumping rounds, records
-        # and the triangle records
-        self.launches = 1 + 21
+        # kernels per step: 1 for the frame; the update's object boxes, leaf
+        # boxes, re-splits, 2 scan kernels, relocation, rotations, paths to the
+        # root, records, triangle records and wide nodes
+        self.launches = 1 + 11
 
     def frame(self, stream_ptr):
         k = self.k % self.PERIOD

@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(128)
     }
   }
   if (!ok || !(big > 1e-15f)) *bad = 1;
-  uint32_t* w = wide + 24 * (size_t)r;
+  uint32_t w[24];
 #pragma unroll
   for (int c = 0; c < 3; ++c) w[c] = __float_as_uint(pb[c]);
   w[3] = __float_as_uint(gs);
@@ -137,6 +137,10 @@ __global__ void __launch_bounds__(128)
   }
   w[20] = meta;
   w[21] = w[22] = w[23] = 0u;
+  uint4* out = reinterpret_cast<uint4*>(wide + 24 * (size_t)r);
+#pragma unroll
+  for (int k = 0; k < 6; ++k)
+    out[k] = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
 }
 
 }  // namespace
