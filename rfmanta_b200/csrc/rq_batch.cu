@@ -60,7 +60,7 @@ struct BatchBinary {
   // so a warp's busy lanes almost always share the query kind: the step is
   // then compiled for that kind (the per-lane form only where kinds meet).
   __device__ __forceinline__ void step(const DevScene& S, Ray& r, Hit& h, bool any, bool live,
-                                       int vote, int& ref) {
+                                       int vote, int& ref, bool slots = false) {
     const unsigned any_m = __ballot_sync(0xffffffffu, live && any);
     const unsigned clo_m = __ballot_sync(0xffffffffu, live && !any);
     if (!live) return;

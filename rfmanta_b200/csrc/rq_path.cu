@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(256)
     }
     if (__all_sync(0xffffffffu, exhausted)) break;
     bool fin = false;
-    walk.step(S, sr, sh, true, p >= 0 && ref != kDone, kPathVote, ref);
+    walk.step(S, sr, sh, true, p >= 0 && ref != kDone, kPathVote, ref, true);
     if (p >= 0 && ref == kDone) {
       if (traced && sh.id < 0) shade_finish(B, p, contrib);
       fin = true;

@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(128) serve_shade_kernel(ServeArgs A, PathBuffe
     if (__all_sync(0xffffffffu, exhausted)) break;
     bool fin = false;
     const DevScene S = walk_scene<Walk>(sm_scenes[scene]);
-    walk.step(S, sr, sh, true, p >= 0 && ref != kDone, kServeVote, ref);
+    walk.step(S, sr, sh, true, p >= 0 && ref != kDone, kServeVote, ref, true);
     if (p >= 0 && ref == kDone) {
       if (traced && sh.id < 0) shade_finish(B, p, contrib);
       fin = true;

@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(256) trace_kernel(const __grid_constant__ DevS
     walk.start(S, r, ANY, h, ref);
   }
   while (__any_sync(0xffffffffu, ref != kDone))
-    walk.step(S, r, h, ANY, ref != kDone, ANY ? kAnyVote : kClosestVote, ref);
+    walk.step(S, r, h, ANY, ref != kDone, ANY ? kAnyVote : kClosestVote, ref, ANY);
   if (i < a.n) store_hit(a, i, h);
 }
 
@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(256)
       }
     }
     if (__all_sync(0xffffffffu, exhausted)) break;
-    walk.step(S, r, h, ANY, idx >= 0 && ref != kDone, ANY ? kAnyVote : kClosestVote, ref);
+    walk.step(S, r, h, ANY, idx >= 0 && ref != kDone, ANY ? kAnyVote : kClosestVote, ref, ANY);
     if (idx >= 0 && ref == kDone) {
       store_hit(a, idx, h);
       idx = -1;

@@ -13,8 +13,10 @@
 //   words 4-7   refs of the four slots (kDone: empty)
 //   words 8-13  box centres x01 x23 y01 y23 z01 z23 (packed 16-bit pairs)
 //   words 14-19 half extents, the same order, padded (rq_wide.cuh)
-//   word 20     4 bits per folded record (r, left, right): axis one-hot and
-//               isLeftCheaper << 3
+//   word 20     a byte per folded record (r, first side, second side): one-hot
+//               of its axis, 3 higher where the side in front is the right one
+// The sides, and the slots within a side, are in any-hit order (the cheaper
+// child, isLeftCheaper, in front).
 //
 // The thread also stores the boxes of r's leaf children (leaf_box) and
 // checks what the walk relies on: finite, nested boxes.
@@ -88,24 +90,33 @@ __global__ void __launch_bounds__(128)
   for (int c = 0; c < 3; ++c) pb[c] = (0.5f * lo[c] + 0.5f * hi[c]) * gs;
   RecBox box[4];
   int ref[4] = {kDone, kDone, kDone, kDone};
-  unsigned meta = (1u << (q3.z & 3)) | (((q3.z >> 2) & 1) << 3);
+  const auto order = [](int meta) {  // its byte of word 20
+    return 1u << ((meta & 3) + ((meta >> 2) & 1 ? 0 : 3));
+  };
+  unsigned meta = order(q3.z);
+  const bool left = (q3.z >> 2) & 1;
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
-    const int c = k ? q3.y : q3.x;
+    const bool is_left = (k == 0) == left;
+    const int c = is_left ? q3.x : q3.y;
+    const RecBox b = side[is_left ? 0 : 1];
     if (c < 0) {
       ref[2 * k] = c;
-      box[2 * k] = side[k];
-      const RecBox& b = side[k];
+      box[2 * k] = b;
       leaf_box[2 * (size_t)(~c)] = make_float4(b.lo[0], b.lo[1], b.lo[2], b.hi[0]);
       leaf_box[2 * (size_t)(~c) + 1] = make_float4(b.hi[1], b.hi[2], 0.f, 0.f);
     } else {
       const float4* s = recs + 4 * (size_t)c;
       const int4 t3 = reinterpret_cast<const int4*>(s)[3];
-      record_boxes(s, box[2 * k], box[2 * k + 1]);
-      ref[2 * k] = t3.x;
-      ref[2 * k + 1] = t3.y;
-      ok = ok && inside(box[2 * k], side[k]) && inside(box[2 * k + 1], side[k]);
-      meta |= ((1u << (t3.z & 3)) | (((t3.z >> 2) & 1) << 3)) << (4 + 4 * k);
+      RecBox x, y;
+      record_boxes(s, x, y);
+      const bool x_first = (t3.z >> 2) & 1;
+      box[2 * k] = x_first ? x : y;
+      box[2 * k + 1] = x_first ? y : x;
+      ref[2 * k] = x_first ? t3.x : t3.y;
+      ref[2 * k + 1] = x_first ? t3.y : t3.x;
+      ok = ok && inside(x, b) && inside(y, b);
+      meta |= order(t3.z) << (8 + 8 * k);
     }
   }
   if (!ok || !(big > 1e-15f)) *bad = 1;

@@ -9,7 +9,8 @@
 // Why the results are the binary walk's, bit for bit:
 //   * the four children are taken in the binary walk's order, which each of
 //     the three folded records fixes by its axis and the ray's direction
-//     signs (closest hit) or its isLeftCheaper flag (any hit);
+//     signs (closest hit) or its isLeftCheaper flag (any hit: the order of the
+//     slots themselves, so kernels of any-hit rays alone swap nothing);
 //   * a 16-bit box only decides what is skipped, and it contains the exact
 //     box by more than all rounding errors (bound below), so no leaf that the
 //     binary walk tests is skipped;
@@ -69,7 +70,8 @@ struct WideRay {
   __half2 p2[3];      // |A|, both halves
   __half2 n2[3];      // -|A|
   float dm;           // |d|max
-  unsigned side;      // bit k: d_k > 0 (closest hit); 8: any hit; for each folded record
+  unsigned side;      // per folded record's byte: bit k: d_k > 0, bit 3 + k: not
+                      // (closest hit); all set: any hit
 };
 
 // Prepares a ray; false when it must take the exact walk.
@@ -93,9 +95,9 @@ __device__ __forceinline__ bool wide_setup(const DevScene& S, const Ray& r, bool
   const float k = __fdividef(-1.f, sum);
 #pragma unroll
   for (int c = 0; c < 3; ++c) w.w[c] = g[c] * k;
-  w.side = 0x111u * (any ? 8u
-                         : (r.d[0] > 0.f ? 1u : 0u) | (r.d[1] > 0.f ? 2u : 0u) |
-                               (r.d[2] > 0.f ? 4u : 0u));
+  const unsigned up =
+      (r.d[0] > 0.f ? 1u : 0u) | (r.d[1] > 0.f ? 2u : 0u) | (r.d[2] > 0.f ? 4u : 0u);
+  w.side = 0x010101u * (any ? 0x3fu : up | (~up & 7u) << 3);
   return ok;
 }
 
@@ -167,8 +169,10 @@ struct WideStack {
 
 // One wide node: the children hit are pushed, last to visit first, and the
 // top of the stack (a child, or an older ref when none was hit) is popped.
+// slots: an any-hit ray, known where the code is compiled - its order is the
+// slots' own.
 __device__ __forceinline__ void wide_visit(const DevScene& S, const Ray& r, const WideRay& w,
-                                           int& ref, WideStack& st) {
+                                           bool slots, int& ref, WideStack& st) {
   const char* p = reinterpret_cast<const char*>(S.wide) + 96 * (size_t)ref;
   const Words8 u0 = load_words8(p), u1 = load_words8(p + 32), u2 = load_words8(p + 64);
   const float gs = __uint_as_float(u0.x[3]);
@@ -197,15 +201,22 @@ __device__ __forceinline__ void wide_visit(const DevScene& S, const Ray& r, cons
   int r0 = (int)u0.x[4], r1 = (int)u0.x[5], r2 = (int)u0.x[6], r3 = (int)u0.x[7];
   keep_hit(near01, far01, r0, r1);
   keep_hit(near23, far23, r2, r3);
-  // the binary order: within each side, then the sides
-  const unsigned m = u2.x[4] & w.side;
-  const bool f0 = (m & 0xfu) != 0u, f1 = (m & 0xf0u) != 0u, f2 = (m & 0xf00u) != 0u;
-  const int a0 = f1 ? r0 : r1, a1 = f1 ? r1 : r0;
-  const int b0 = f2 ? r2 : r3, b1 = f2 ? r3 : r2;
-  st.push_hit(f0 ? b1 : a1);
-  st.push_hit(f0 ? b0 : a0);
-  st.push_hit(f0 ? a1 : b1);
-  st.push_hit(f0 ? a0 : b0);
+  if (slots) {
+    st.push_hit(r3);
+    st.push_hit(r2);
+    st.push_hit(r1);
+    st.push_hit(r0);
+  } else {
+    // the binary order: within each side, then the sides
+    const unsigned m = u2.x[4] & w.side;
+    const bool f0 = (m & 0xffu) != 0u, f1 = (m & 0xff00u) != 0u, f2 = (m & 0xff0000u) != 0u;
+    const int a0 = f1 ? r0 : r1, a1 = f1 ? r1 : r0;
+    const int b0 = f2 ? r2 : r3, b1 = f2 ? r3 : r2;
+    st.push_hit(f0 ? b1 : a1);
+    st.push_hit(f0 ? b0 : a0);
+    st.push_hit(f0 ? a1 : b1);
+    st.push_hit(f0 ? a0 : b0);
+  }
   ref = st.pop();
 }
 
@@ -217,7 +228,7 @@ __device__ __forceinline__ void wide_leaf(const DevScene& S, Ray& r, Hit& h, boo
   const int first = ~ref;
   const float4* p = S.tris + 3 * (size_t)first;
   bool in_box = false;
-  for (;;) {
+  for (int pos = first;; ++pos) {
     bool last;
     const float t_in = r.minT;
     Hit n;
@@ -235,7 +246,7 @@ __device__ __forceinline__ void wide_leaf(const DevScene& S, Ray& r, Hit& h, boo
         r.minT = t_hit;
       }
       h = n;
-      h.pos = (int)((p - S.tris) / 3);
+      h.pos = pos;
       if (any) {
         ref = kDone;
         return;
@@ -287,20 +298,21 @@ __device__ __forceinline__ void wide_start(const DevScene& S, Ray& r, bool any, 
 // or at their end, then the waiting leaves.  Called by all 32 lanes.
 template <int KIND>
 __device__ __forceinline__ void wide_step(const DevScene& S, Ray& r, const WideRay& w, Hit& h,
-                                          bool any, bool live, int vote, int& ref,
-                                          WideStack& st) {
+                                          bool any, bool live, int vote, bool slots,
+                                          int& ref, WideStack& st) {
   const int stop = max(0, __popc(__ballot_sync(0xffffffffu, live)) - vote);
   while (__popc(__ballot_sync(0xffffffffu, live && (unsigned)ref < (unsigned)kDone)) > stop) {
 #pragma unroll
     for (int k = 0; k < kWideVisits; ++k)
-      if (live && (unsigned)ref < (unsigned)kDone) wide_visit(S, r, w, ref, st);
+      if (live && (unsigned)ref < (unsigned)kDone) wide_visit(S, r, w, slots, ref, st);
   }
   if (live && ref < 0) wide_leaf<KIND>(S, r, h, any, ref, st);
 }
 
 // The two walks behind one interface, for kernels whose warps keep one ray per
 // lane in flight: init once, start per ray (ref = kDone when it is finished
-// already), step by the whole warp with `live` where ref != kDone.
+// already), step by the whole warp with `live` where ref != kDone (slots: every
+// ray is an any-hit ray, said where the code is compiled).
 
 // Binary walk over the node records, R stack entries in registers; a step of
 // a lane runs to its next leaf and through it.
@@ -319,7 +331,7 @@ struct BinaryWalk {
     if (STATS) cnt.boxes += 1;
   }
   __device__ __forceinline__ void step(const DevScene& S, Ray& r, Hit& h, bool any, bool live,
-                                       int vote, int& ref) {
+                                       int vote, int& ref, bool slots = false) {
     if (live) step_dyn<KIND, R, STATS>(S, r, h, ref, st, any, &cnt);
   }
 };
@@ -339,8 +351,8 @@ struct WideWalk {
     wide_start<KIND>(S, r, any, w, h, ref, st);
   }
   __device__ __forceinline__ void step(const DevScene& S, Ray& r, Hit& h, bool any, bool live,
-                                       int vote, int& ref) {
-    wide_step<KIND>(S, r, w, h, any, live, vote, ref, st);
+                                       int vote, int& ref, bool slots = false) {
+    wide_step<KIND>(S, r, w, h, any, live, vote, slots, ref, st);
   }
 };
 
