@@ -60,8 +60,12 @@ constexpr int kPathVote = 16;
 
 // Walk: the wide walk, or the binary one with its options (statistics,
 // register stack entries) - rq_wide.cuh.
+// Registers are capped so that seven (extend) and eight (shade) 128-thread
+// blocks fit an SM: uncapped the shade stage took 78-80 and six blocks (frame
+// 9.20 ms; shade at 72 / 64 registers 9.02 / 8.81, extend at 72 too 8.91 / 8.68,
+// extend at 56 spills: 9.04).
 template <class Walk>
-__global__ void __launch_bounds__(256)
+__global__ void __maxnreg__(72)
     path_extend_persistent_kernel(DevScene S, PathParams P, PathBuffers B, int depth, int n0,
                                   int refill) {
   extern __shared__ int2 smem_stack[];
@@ -123,7 +127,7 @@ __global__ void __launch_bounds__(256)
 // needed) it applies shade_finish and the survivors are compacted into the
 // next queue at the warp's common point, one atomic per warp.
 template <class Walk>
-__global__ void __launch_bounds__(256)
+__global__ void __maxnreg__(64)
     path_shade_persistent_kernel(DevScene S, PathParams P, PathBuffers B, int depth, int n0,
                                  int refill) {
   extern __shared__ int2 smem_stack[];
