@@ -689,7 +689,9 @@ typedef struct {
                                      do_ambient_on_maxdepth) */
   int n_materials;
   const float* material_rgb;      /* host: n_materials x (r, g, b) */
-  int chunk_paths;                /* paths per wavefront pass, 0 = 4Mi */
+  int chunk_paths;                /* paths per wavefront pass, 0 = the whole frame, or
+                                     equal parts of at most 32Mi paths (77 bytes of
+                                     device memory each; smaller where that is short) */
   rq_environment environment;     /* zero = constant ambient and background;
                                      EyeAmbient at the last bounce sees the
                                      direction sampled there, as the

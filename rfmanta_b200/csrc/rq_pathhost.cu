@@ -14,6 +14,12 @@
 
 namespace rq {
 
+// Paths per wavefront pass when the caller leaves it to the library, and where
+// it stops trying smaller passes.  The 1280x720x16 frame in passes of 2 / 4 / 8 /
+// 16 Mi paths: 10.57 / 8.68 / 7.91 / 7.33 ms; 77 bytes of state per path.
+constexpr long long kAutoChunk = 32LL << 20;
+constexpr long long kLeastChunk = 1LL << 20;
+
 struct PathScratch {
   size_t capacity = 0;
   PathBuffers B{};
@@ -32,6 +38,23 @@ struct PathScratch {
     B.alive = nullptr;
     B.pos = B.prim = B.queue[0] = B.queue[1] = B.counters = B.tile_counts = nullptr;
     capacity = 0;
+  }
+  bool allocate(size_t C) {
+    auto get = [](auto** q, size_t n) {
+      return cudaMalloc(reinterpret_cast<void**>(q), std::max<size_t>(n, 1) * sizeof(**q)) ==
+             cudaSuccess;
+    };
+    free_paths();
+    if (!get(&B.o, 3 * C) || !get(&B.d, 3 * C) || !get(&B.imp, 3 * C) || !get(&B.rad, 3 * C) ||
+        !get(&B.rng, C) || !get(&B.t, C) || !get(&B.pos, C) || !get(&B.prim, C) ||
+        !get(&B.queue[0], C) || !get(&B.queue[1], C) || !get(&B.counters, kPathCounters) ||
+        !get(&B.alive, C) || !get(&B.tile_counts, C / 4096 + 2)) {
+      free_paths();
+      return false;
+    }
+    capacity = C;
+    B.capacity = C;
+    return true;
   }
   ~PathScratch() {
     free_paths();
@@ -96,25 +119,23 @@ static int path_prepare(Scene* s, const rq_path_params* p, PathParams& P, long l
   for (int c = 0; c < 3; ++c) P.light_normal[c] = n[c] * sc;
   P.light_inv_area = (float)1 / l;
   total = (long long)p->xres * p->yres * p->spp;
-  long long ch = p->chunk_paths > 0 ? p->chunk_paths : (4LL << 20);
-  ch = std::max<long long>(ch / p->spp, 1) * p->spp;  // whole pixels per chunk
-  chunk = (int)std::min<long long>(ch, total);
   if (!s->paths) s->paths = new PathScratch();
   PathScratch* ps = s->paths;
-  if (ps->capacity < (size_t)chunk) {
-    ps->free_paths();
-    const size_t C = (size_t)chunk;
-    PathBuffers& B = ps->B;
-    if (!palloc(&B.o, 3 * C) || !palloc(&B.d, 3 * C) || !palloc(&B.imp, 3 * C) ||
-        !palloc(&B.rad, 3 * C) || !palloc(&B.rng, C) || !palloc(&B.t, C) ||
-        !palloc(&B.pos, C) || !palloc(&B.prim, C) || !palloc(&B.queue[0], C) ||
-        !palloc(&B.queue[1], C) || !palloc(&B.counters, kPathCounters) ||
-        !palloc(&B.alive, C) || !palloc(&B.tile_counts, C / 4096 + 2)) {
-      ps->free_paths();
+  // 0: the whole frame, or equal parts of at most kAutoChunk paths - every
+  // part pays the ends of its persistent stages again (two per bounce), where
+  // the SMs run out of paths.  Parts are made smaller while memory is short.
+  long long parts = (total + kAutoChunk - 1) / kAutoChunk;
+  for (;;) {
+    long long ch = p->chunk_paths > 0 ? p->chunk_paths : (total + parts - 1) / parts;
+    // whole pixels per chunk
+    ch = std::max<long long>((p->chunk_paths > 0 ? ch : ch + p->spp - 1) / p->spp, 1) * p->spp;
+    chunk = (int)std::min<long long>(ch, total);
+    if (ps->capacity >= (size_t)chunk) break;
+    if (ps->allocate((size_t)chunk)) break;
+    cudaGetLastError();
+    if (p->chunk_paths > 0 || chunk <= kLeastChunk)
       return pfail(RQ_ERR_OOM, "path state allocation failed");
-    }
-    ps->capacity = C;
-    B.capacity = C;
+    parts *= 2;
   }
   if (!ps->counts && !palloc(&ps->counts, 2)) return pfail(RQ_ERR_OOM, "counter allocation");
   const float* mrgb = p->material_rgb;
