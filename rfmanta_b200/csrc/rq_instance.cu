@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -36,7 +37,7 @@ static float bits_as_float(int32_t i) {
 
 // ------------------------------------------------------------ queries ----
 
-template <int KIND, bool ANY>
+template <int KIND, bool ANY, bool WIDE>
 __global__ void __launch_bounds__(128)
     trace2_kernel(DevScene T, const DevScene* blas, RayArgs a, int32_t* inst) {
   extern __shared__ int2 smem_stack[];
@@ -53,7 +54,7 @@ __global__ void __launch_bounds__(128)
   r.minT = __ldg(a.tmax + i);
   Hit h;
   int ih, bh;
-  trace_two_level<KIND, ANY>(T, blas, r, h, ih, bh, smem_stack + threadIdx.x, blockDim.x);
+  trace_two_level<KIND, ANY, false, WIDE>(T, blas, r, h, ih, bh, smem_stack + threadIdx.x, blockDim.x);
   if (a.t) a.t[i] = h.t;
   if (a.prim) a.prim[i] = h.id;
   if (a.u) a.u[i] = h.u;
@@ -61,28 +62,48 @@ __global__ void __launch_bounds__(128)
   if (inst) inst[i] = ih;
 }
 
+// Stack bytes per block of a two-level walk: the top-level entries, then the
+// inner scenes' (their own column, or the same one).
+static size_t two_level_bytes(const Scene& s, int block, bool wide) {
+  const int top = s.dev().depth;
+  return wide ? (size_t)top * block * sizeof(int2) + stack_bytes(s.max_blas_depth, block, true)
+              : (size_t)(top + s.max_blas_depth + 1) * block * sizeof(int2);
+}
+
+bool Scene::inner_wide() const {
+  // rays reach an instance from anywhere in the scene and some way outside:
+  // the inner scenes' origin limits (kWideOrigin of their sizes) must cover
+  // four times the scene, or too many of them would take the exact walk
+  float size = 0.f;
+  for (int c = 0; c < 3; ++c)
+    size = std::max(size, std::max(std::fabs(root_lo[c]), std::fabs(root_hi[c])));
+  for (const Scene* b : blas)
+    if (!b->dev().wide || kWideOrigin * b->wide_extent < 4.f * size) return false;
+  return instanced;
+}
+
 cudaError_t launch_trace2(const Scene& s, const RayArgs& a, bool anyhit, int32_t* inst,
                           cudaStream_t st) {
   if (a.n <= 0) return cudaSuccess;
   const DevScene T = s.dev();
   const int bs = 128;
-  const size_t smem = (size_t)(T.depth + s.max_blas_depth + 1) * bs * sizeof(int2);
+  const bool wide = s.inner_wide();
+  const size_t smem = two_level_bytes(s, bs, wide);
   const int grid = (a.n + bs - 1) / bs;
-  const void* f = s.tri_kind == kWald
-                      ? (anyhit ? (const void*)trace2_kernel<kWald, true>
-                                : (const void*)trace2_kernel<kWald, false>)
-                      : (anyhit ? (const void*)trace2_kernel<kKS, true>
-                                : (const void*)trace2_kernel<kKS, false>);
+  const void* f =
+      s.tri_kind == kWald
+          ? (anyhit ? (wide ? (const void*)trace2_kernel<kWald, true, true>
+                            : (const void*)trace2_kernel<kWald, true, false>)
+                    : (wide ? (const void*)trace2_kernel<kWald, false, true>
+                            : (const void*)trace2_kernel<kWald, false, false>))
+          : (anyhit ? (wide ? (const void*)trace2_kernel<kKS, true, true>
+                            : (const void*)trace2_kernel<kKS, true, false>)
+                    : (wide ? (const void*)trace2_kernel<kKS, false, true>
+                            : (const void*)trace2_kernel<kKS, false, false>));
   if (smem > 48 * 1024)
     cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (s.tri_kind == kWald) {
-    if (anyhit) trace2_kernel<kWald, true><<<grid, bs, smem, st>>>(T, s.d_blas, a, inst);
-    else trace2_kernel<kWald, false><<<grid, bs, smem, st>>>(T, s.d_blas, a, inst);
-  } else {
-    if (anyhit) trace2_kernel<kKS, true><<<grid, bs, smem, st>>>(T, s.d_blas, a, inst);
-    else trace2_kernel<kKS, false><<<grid, bs, smem, st>>>(T, s.d_blas, a, inst);
-  }
-  return cudaGetLastError();
+  void* args[] = {(void*)&T, (void*)&s.d_blas, (void*)&a, (void*)&inst};
+  return cudaLaunchKernel(f, dim3(grid), dim3(bs), args, smem, st);
 }
 
 // Lays out the top-level tree of an instanced scene: node records as for a
@@ -295,6 +316,25 @@ struct SampleBufs {
   int32_t* tiles;   // compaction scratch
 };
 
+// A lane of these kernels traces its own sample to the end, nested in the
+// two-level walk, so a warp waits for its slowest ray: what helps is work the
+// lanes share.  Over the 1920x1080x4 two-level frame the inner scenes' wide
+// nodes and tiles of pixels took 2.55 -> 2.14 ms (tiles alone 2.46); warps that
+// step both levels together and refill, with separate shadow and shade stages,
+// 2.69.
+//
+// Sample of work item k: a warp's 32 items are the samples of a tile of pixels
+// (8x4, 4x2 or 2x1 at 1, 4 or 16 samples) where those tiles cover the image, else
+// 32 consecutive samples.
+__device__ __forceinline__ int item_sample(const FrameParams& P, const SampleParams& Q, int k) {
+  const int tw = Q.spp == 1 ? 8 : Q.spp == 4 ? 4 : 2, th = Q.spp == 1 ? 4 : Q.spp == 4 ? 2 : 1;
+  if (Q.spp * tw * th != 32 || P.xres % tw || P.yres % th) return k;
+  const int tile = k >> 5, l = k & 31, n = P.xres / tw;
+  const int px = l / Q.spp, sm = l - px * Q.spp;
+  const int x = (tile % n) * tw + px % tw, y = (tile / n) * th + px / tw;
+  return (y * P.xres + x) * Q.spp + sm;
+}
+
 __device__ __forceinline__ void sample_ray(const FrameParams& P, const SampleParams& Q,
                                            long long item, Ray& r) {
   const long long pix = item / Q.spp;
@@ -329,13 +369,24 @@ __device__ __forceinline__ void sample_ray(const FrameParams& P, const SamplePar
   r.minT = kMaxT;
 }
 
-template <int KIND, bool TWO, bool ANY, bool STATS>
+template <int KIND, bool TWO, bool ANY, bool STATS, bool WIDE>
 __device__ __forceinline__ void scene_trace(const DevScene& S, const DevScene* blas, Ray& r,
                                             Hit& h, int& bh, int2* stk, int stride,
                                             Counts* cnt) {
   if (TWO) {
     int ih;
-    trace_two_level<KIND, ANY, STATS>(S, blas, r, h, ih, bh, stk, stride, cnt);
+    trace_two_level<KIND, ANY, STATS, WIDE>(S, blas, r, h, ih, bh, stk, stride, cnt);
+  } else if (WIDE) {
+    WideStack st;
+    st.init(reinterpret_cast<int*>(stk - threadIdx.x) + threadIdx.x, stride);
+    WideRay w;
+    int ref;
+    wide_start<KIND>(S, r, ANY, w, h, ref, st);
+    while (ref != kDone) {
+      while ((unsigned)ref < (unsigned)kDone) wide_visit(S, r, w, ANY, ref, st);
+      if (ref < 0) wide_leaf<KIND>(S, r, h, ANY, ref, st);
+    }
+    bh = -1;
   } else {
     int ref, sp;
     if (STATS) cnt->boxes += 1;
@@ -357,7 +408,7 @@ __device__ __forceinline__ void add_counts(unsigned long long* dst, int a, int b
   }
 }
 
-template <int KIND, bool TWO, bool STATS>
+template <int KIND, bool TWO, bool STATS, bool WIDE>
 __global__ void __launch_bounds__(128)
     frame_primary_kernel(DevScene S, const DevScene* blas, FrameParams P, SampleParams Q,
                          SampleBufs B, int n_items, unsigned long long* stats) {
@@ -370,7 +421,8 @@ __global__ void __launch_bounds__(128)
     if (lane == 0) base = atomicAdd(&B.counters[1], 32);
     base = __shfl_sync(0xffffffffu, base, 0);
     if (base >= n_items) break;
-    const int it = base + (int)lane;
+    const int k = base + (int)lane;
+    const int it = k < n_items ? item_sample(P, Q, k) : n_items;
     bool hit = false;
     Counts cnt;
     if (it < n_items) {
@@ -378,7 +430,7 @@ __global__ void __launch_bounds__(128)
       sample_ray(P, Q, it, r);
       Hit h;
       int bh;
-      scene_trace<KIND, TWO, false, STATS>(S, blas, r, h, bh, smem_stack + threadIdx.x,
+      scene_trace<KIND, TWO, false, STATS, WIDE>(S, blas, r, h, bh, smem_stack + threadIdx.x,
                                            blockDim.x, &cnt);
       B.t[it] = h.t;
       B.prim[it] = h.id;
@@ -394,7 +446,7 @@ __global__ void __launch_bounds__(128)
     // the shade queue is compacted in sample order afterwards, so that the
     // shade stage's warps take neighbouring samples whatever order the
     // primary warps finished in
-    if (it < n_items) B.hit[it] = hit ? 1 : 0;
+    if (k < n_items) B.hit[k] = hit ? 1 : 0;
     if (STATS) add_counts(stats, cnt.boxes, cnt.tris);
   }
 }
@@ -404,7 +456,7 @@ __global__ void __launch_bounds__(128)
 // local colour in col, the face-forward normal and hit point for a
 // reflection.  Returns the material's reflectivity (0 unless a reflective
 // Phong).
-template <int KIND, bool TWO, bool STATS>
+template <int KIND, bool TWO, bool STATS, bool WIDE>
 __device__ __forceinline__ float shade_hit(const DevScene& S, const DevScene* blas,
                                            const FrameParams& P, const Ray& r, float t,
                                            int prim, int pos, int bh, int2* stk, int stride,
@@ -448,7 +500,7 @@ __device__ __forceinline__ float shade_hit(const DevScene& S, const DevScene* bl
     ++nshadow;
     Hit sh;
     int sb;
-    scene_trace<KIND, TWO, true, STATS>(S, blas, s, sh, sb, stk, stride, cnt);
+    scene_trace<KIND, TWO, true, STATS, WIDE>(S, blas, s, sh, sb, stk, stride, cnt);
     if (sh.id >= 0) continue;
     const float sum = fadd(fadd(fmul(sd[0], sd[0]), fmul(sd[1], sd[1])), fmul(sd[2], sd[2]));
     const float scale = fdiv(1.f, __fsqrt_rn(sum));
@@ -493,7 +545,7 @@ __device__ __forceinline__ float shade_hit(const DevScene& S, const DevScene* bl
 // chain is then folded from its end, colour = local + child x reflectivity,
 // in the reference's order (a reflection cut off by importance adds black
 // x reflectivity).
-template <int KIND, bool TWO, bool STATS, bool REFL>
+template <int KIND, bool TWO, bool STATS, bool WIDE, bool REFL>
 __global__ void __launch_bounds__(128)
     frame_shade_kernel(DevScene S, const DevScene* blas, FrameParams P, SampleParams Q,
                        SampleBufs B, unsigned long long* stats) {
@@ -511,11 +563,11 @@ __global__ void __launch_bounds__(128)
     int nshadow = 0;
     Counts cnt;
     if (qi < nq) {
-      const int it = B.queue[qi];
+      const int it = item_sample(P, Q, B.queue[qi]);
       Ray r;
       sample_ray(P, Q, it, r);
       float col[3], ffn[3], hp[3];
-      const float refl = shade_hit<KIND, TWO, STATS>(S, blas, P, r, B.t[it], B.prim[it],
+      const float refl = shade_hit<KIND, TWO, STATS, WIDE>(S, blas, P, r, B.t[it], B.prim[it],
                                                      B.pos[it], B.blas[it], stk, stride, &cnt,
                                                      nshadow, col, ffn, hp);
       if (!REFL || refl == 0.f || P.max_depth <= 0) {
@@ -551,7 +603,7 @@ __global__ void __launch_bounds__(128)
           q.minT = kMaxT;
           Hit qh;
           int qb;
-          scene_trace<KIND, TWO, false, STATS>(S, blas, q, qh, qb, stk, stride, &cnt);
+          scene_trace<KIND, TWO, false, STATS, WIDE>(S, blas, q, qh, qb, stk, stride, &cnt);
           ++depth;
 #pragma unroll
           for (int c = 0; c < 3; ++c) imp[c] = ci[c];
@@ -560,7 +612,7 @@ __global__ void __launch_bounds__(128)
             rf[depth] = 0.f;
             break;
           }
-          rf[depth] = shade_hit<KIND, TWO, STATS>(S, blas, P, q, qh.t, qh.id, qh.pos, qb, stk,
+          rf[depth] = shade_hit<KIND, TWO, STATS, WIDE>(S, blas, P, q, qh.t, qh.id, qh.pos, qb, stk,
                                                   stride, &cnt, nshadow, loc[depth], ffn, hp);
 #pragma unroll
           for (int c = 0; c < 3; ++c) d[c] = q.d[c];
@@ -593,17 +645,18 @@ __global__ void frame_resolve_kernel(SampleParams Q, SampleBufs B, int npix, flo
   }
 }
 
-template <int KIND, bool TWO, bool STATS>
+template <int KIND, bool TWO, bool STATS, bool WIDE>
 static cudaError_t frame_go(const Scene& s, const FrameParams& P, const SampleParams& Q,
                             const SampleBufs& B, int npix, float* rgb, cudaStream_t st,
                             const cudaEvent_t* ev, int nev) {
   const DevScene S = s.dev();
   const int bs = 128;
-  const size_t smem = (size_t)(S.depth + (TWO ? s.max_blas_depth : 0) + 1) * bs * sizeof(int2);
+  const size_t smem =
+      TWO ? two_level_bytes(s, bs, WIDE) : stack_bytes(S.depth + 1, bs, WIDE);
   const bool refl = P.refl != nullptr;
-  const void* f1 = (const void*)frame_primary_kernel<KIND, TWO, STATS>;
-  const void* f2 = refl ? (const void*)frame_shade_kernel<KIND, TWO, STATS, true>
-                        : (const void*)frame_shade_kernel<KIND, TWO, STATS, false>;
+  const void* f1 = (const void*)frame_primary_kernel<KIND, TWO, STATS, WIDE>;
+  const void* f2 = refl ? (const void*)frame_shade_kernel<KIND, TWO, STATS, WIDE, true>
+                        : (const void*)frame_shade_kernel<KIND, TWO, STATS, WIDE, false>;
   if (smem > 48 * 1024) {
     cudaFuncSetAttribute(f1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     cudaFuncSetAttribute(f2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -617,17 +670,17 @@ static cudaError_t frame_go(const Scene& s, const FrameParams& P, const SamplePa
   if (e == cudaSuccess) e = cudaMemsetAsync(B.shadow, 0, sizeof(unsigned long long), st);
   if (e != cudaSuccess) return e;
   if (nev > 0) cudaEventRecord(ev[0], st);
-  frame_primary_kernel<KIND, TWO, STATS>
+  frame_primary_kernel<KIND, TWO, STATS, WIDE>
       <<<std::max(1, std::min(grid, (n_items + bs - 1) / bs)), bs, smem, st>>>(
           S, s.d_blas, P, Q, B, n_items, s.stats);
   e = launch_flag_compaction(B.hit, n_items, B.tiles, &B.counters[0], B.queue, st);
   if (e != cudaSuccess) return e;
   if (nev > 1) cudaEventRecord(ev[1], st);
   if (refl)
-    frame_shade_kernel<KIND, TWO, STATS, true><<<grid, bs, smem, st>>>(S, s.d_blas, P, Q, B,
+    frame_shade_kernel<KIND, TWO, STATS, WIDE, true><<<grid, bs, smem, st>>>(S, s.d_blas, P, Q, B,
                                                                       s.stats);
   else
-    frame_shade_kernel<KIND, TWO, STATS, false><<<grid, bs, smem, st>>>(S, s.d_blas, P, Q, B,
+    frame_shade_kernel<KIND, TWO, STATS, WIDE, false><<<grid, bs, smem, st>>>(S, s.d_blas, P, Q, B,
                                                                        s.stats);
   if (nev > 2) cudaEventRecord(ev[2], st);
   frame_resolve_kernel<<<std::max(1, std::min(grid, (npix + 255) / 256)), 256, 0, st>>>(Q, B, npix, rgb);
@@ -638,10 +691,15 @@ static cudaError_t frame_go(const Scene& s, const FrameParams& P, const SamplePa
 template <int KIND, bool TWO>
 static cudaError_t frame_go_any(const Scene& s, const FrameParams& P, const SampleParams& Q,
                                 const SampleBufs& B, int npix, float* rgb, cudaStream_t st) {
-  return s.stats ? frame_go<KIND, TWO, true>(s, P, Q, B, npix, rgb, st, s.stage_events,
-                                             s.n_stage_events)
-                 : frame_go<KIND, TWO, false>(s, P, Q, B, npix, rgb, st, s.stage_events,
-                                              s.n_stage_events);
+  // counted tests are the binary walk's
+  if (s.stats)
+    return frame_go<KIND, TWO, true, false>(s, P, Q, B, npix, rgb, st, s.stage_events,
+                                            s.n_stage_events);
+  if (TWO ? s.inner_wide() : s.dev().wide != nullptr)
+    return frame_go<KIND, TWO, false, true>(s, P, Q, B, npix, rgb, st, s.stage_events,
+                                            s.n_stage_events);
+  return frame_go<KIND, TWO, false, false>(s, P, Q, B, npix, rgb, st, s.stage_events,
+                                           s.n_stage_events);
 }
 
 // Scratch of the supersampled frame, owned by the scene.

@@ -9,13 +9,15 @@
 // DynBVH::intersect and accepts the result through RayPacket::hit.
 #pragma once
 
-#include "rq_traverse.cuh"
+#include "rq_wide.cuh"
 
 namespace rq {
 
 // With STATS, cnt counts box tests (two per top-level record, one per root
-// box, the instance's included) and triangle tests.
-template <int KIND, bool ANY, bool STATS = false>
+// box, the instance's included) and triangle tests.  WIDE: the inner scenes
+// are walked over their wide nodes, on a column of their own behind the
+// top-level entries (every inner tree has them).
+template <int KIND, bool ANY, bool STATS = false, bool WIDE = false>
 __device__ __forceinline__ void trace_two_level(const DevScene& T, const DevScene* blas,
                                                 Ray& r, Hit& h, int& inst_hit, int& blas_hit,
                                                 int2* stk, int stride, Counts* cnt = nullptr) {
@@ -33,6 +35,14 @@ __device__ __forceinline__ void trace_two_level(const DevScene& T, const DevScen
   int ref = T.root_ref;
   int sp = 0;
   const bool fast = inv_finite(r);
+  WideStack wst;
+  WideRay w;
+  bool wide_ok = false;
+  if (WIDE) {
+    wst.init(reinterpret_cast<int*>(stk - threadIdx.x + (size_t)T.depth * stride) + threadIdx.x,
+             stride);
+    wide_ok = wide_setup(INFINITY, r, ANY, w);  // (the origin is checked per instance)
+  }
   for (;;) {
     while (ref >= 0 && ref != kDone) {
       if (STATS) cnt->boxes += 2;
@@ -86,8 +96,27 @@ __device__ __forceinline__ void trace_two_level(const DevScene& T, const DevScen
       int lref, lsp;
       if (STATS) cnt->boxes += 1;
       start_ray(S, lr, lh, lref, lsp);
-      while (lref != kDone)
-        step<KIND, ANY, STATS>(S, lr, lh, lref, lsp, stk + sp * stride, stride, cnt);
+      if (WIDE) {
+        const float lim = S.origin_limit;
+        if (lref != kDone && !(wide_ok && fabsf(lr.o[0]) <= lim && fabsf(lr.o[1]) <= lim &&
+                               fabsf(lr.o[2]) <= lim)) {
+          lh = wide_trace_exact<KIND, ANY>(S.nodes, S.tris, lref, lr);
+          lr.minT = lh.id >= 0 ? lh.t : lr.minT;
+          lref = kDone;
+        }
+        wst.reset();
+        DevScene L;
+        L.wide = S.wide;
+        L.tris = S.tris;
+        L.leaf_box = S.leaf_box;
+        while (lref != kDone) {
+          while ((unsigned)lref < (unsigned)kDone) wide_visit(L, lr, w, ANY, lref, wst);
+          if (lref < 0) wide_leaf<KIND>(L, lr, lh, ANY, lref, wst);
+        }
+      } else {
+        while (lref != kDone)
+          step<KIND, ANY, STATS>(S, lr, lh, lref, lsp, stk + sp * stride, stride, cnt);
+      }
       if (lh.id >= 0) {
         r.minT = lr.minT;
         h = lh;

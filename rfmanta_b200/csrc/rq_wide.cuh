@@ -74,8 +74,9 @@ struct WideRay {
                       // (closest hit); all set: any hit
 };
 
-// Prepares a ray; false when it must take the exact walk.
-__device__ __forceinline__ bool wide_setup(const DevScene& S, const Ray& r, bool any,
+// Prepares a ray; false when it must take the exact walk in a tree with this
+// origin limit.
+__device__ __forceinline__ bool wide_setup(float origin_limit, const Ray& r, bool any,
                                            WideRay& w) {
   const float ax = fabsf(r.d[0]), ay = fabsf(r.d[1]), az = fabsf(r.d[2]);
   w.dm = fmaxf(fmaxf(ax, ay), az);
@@ -85,7 +86,7 @@ __device__ __forceinline__ bool wide_setup(const DevScene& S, const Ray& r, bool
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     w.A[c] = w.dm * r.inv[c];
-    ok = ok && fabsf(w.A[c]) <= kWideSlope && fabsf(r.o[c]) <= S.origin_limit;
+    ok = ok && fabsf(w.A[c]) <= kWideSlope && fabsf(r.o[c]) <= origin_limit;
     g[c] = r.d[c] * rd;
     sum = __fmaf_rn(g[c], g[c], sum);
     w.a2[c] = __float2half2_rn(w.A[c]);
@@ -283,7 +284,7 @@ __device__ __noinline__ Hit wide_trace_exact(const float4* nodes, const float4* 
 template <int KIND>
 __device__ __forceinline__ void wide_start(const DevScene& S, Ray& r, bool any, WideRay& w,
                                            Hit& h, int& ref, WideStack& st) {
-  const bool ok = wide_setup(S, r, any, w);
+  const bool ok = wide_setup(S.origin_limit, r, any, w);
   int sp;
   start_ray(S, r, h, ref, sp);
   if (!ok && ref != kDone) {
