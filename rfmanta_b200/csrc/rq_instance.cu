@@ -409,7 +409,7 @@ __device__ __forceinline__ void add_counts(unsigned long long* dst, int a, int b
 }
 
 template <int KIND, bool TWO, bool STATS, bool WIDE>
-__global__ void __launch_bounds__(128)
+__global__ void __maxnreg__(72)
     frame_primary_kernel(DevScene S, const DevScene* blas, FrameParams P, SampleParams Q,
                          SampleBufs B, int n_items, unsigned long long* stats) {
   extern __shared__ int2 smem_stack[];
@@ -546,7 +546,7 @@ __device__ __forceinline__ float shade_hit(const DevScene& S, const DevScene* bl
 // in the reference's order (a reflection cut off by importance adds black
 // x reflectivity).
 template <int KIND, bool TWO, bool STATS, bool WIDE, bool REFL>
-__global__ void __launch_bounds__(128)
+__global__ void __maxnreg__(72)
     frame_shade_kernel(DevScene S, const DevScene* blas, FrameParams P, SampleParams Q,
                        SampleBufs B, unsigned long long* stats) {
   extern __shared__ int2 smem_stack[];

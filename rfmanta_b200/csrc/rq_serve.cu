@@ -103,8 +103,10 @@ constexpr int kServeVote = 16;  // wide walk, as the path stages
 // slot's ray in flight in that slot's request scene; warps refill idle lanes
 // with one atomic on the bounce's work counter (as path_extend_persistent_
 // kernel does for a single frame).
+// Registers as the path stages' (uncapped 72 and 96: 5.34 ms of device time for
+// twelve mixed requests; 72 / 80, 72 / 72, 72 / 64: 4.94, 4.71, 5.00).
 template <class Walk>
-__global__ void __launch_bounds__(128) serve_extend_kernel(ServeArgs A, PathBuffers B, int depth) {
+__global__ void __maxnreg__(72) serve_extend_kernel(ServeArgs A, PathBuffers B, int depth) {
   extern __shared__ int2 smem_stack[];
   __shared__ DevScene sm_scenes[kMaxServeScenes];
   stage_scenes(A, sm_scenes);
@@ -159,7 +161,7 @@ __global__ void __launch_bounds__(128) serve_extend_kernel(ServeArgs A, PathBuff
 // shade_finish per lane, survivors compacted into the next queue at the
 // warp's common point.
 template <class Walk>
-__global__ void __launch_bounds__(128) serve_shade_kernel(ServeArgs A, PathBuffers B, int depth) {
+__global__ void __maxnreg__(72) serve_shade_kernel(ServeArgs A, PathBuffers B, int depth) {
   extern __shared__ int2 smem_stack[];
   __shared__ DevScene sm_scenes[kMaxServeScenes];
   stage_scenes(A, sm_scenes);
