@@ -29,14 +29,24 @@ struct PathScratch {
   float* d_rgb = nullptr;
   size_t rgb_pix = 0;
   cudaStream_t stream = nullptr;
-  void free_paths() {
+  // A frame recorded into a CUDA graph holds B's pointers, so such buffers are
+  // kept until the scene goes when a larger frame replaces them (at most one
+  // set per recorded size: capacities only grow).
+  bool recorded = false;
+  std::vector<PathBuffers> retired;
+  static void free_buffers(PathBuffers& B) {
     cudaFree(B.o); cudaFree(B.d); cudaFree(B.imp); cudaFree(B.rad); cudaFree(B.rng);
     cudaFree(B.t); cudaFree(B.pos); cudaFree(B.prim); cudaFree(B.queue[0]);
     cudaFree(B.queue[1]); cudaFree(B.counters); cudaFree(B.alive); cudaFree(B.tile_counts);
-    B.o = B.d = B.imp = B.rad = B.t = nullptr;
-    B.rng = nullptr;
-    B.alive = nullptr;
-    B.pos = B.prim = B.queue[0] = B.queue[1] = B.counters = B.tile_counts = nullptr;
+    B = PathBuffers{};
+  }
+  void free_paths() {
+    if (recorded)
+      retired.push_back(B);
+    else
+      free_buffers(B);
+    B = PathBuffers{};
+    recorded = false;
     capacity = 0;
   }
   bool allocate(size_t C) {
@@ -57,7 +67,8 @@ struct PathScratch {
     return true;
   }
   ~PathScratch() {
-    free_paths();
+    free_buffers(B);
+    for (PathBuffers& b : retired) free_buffers(b);
     cudaFree(materials);
     cudaFree(counts);
     cudaFree(d_rgb);
@@ -77,8 +88,17 @@ static bool palloc(T** p, size_t n) {
   return cudaMalloc(reinterpret_cast<void**>(p), std::max<size_t>(n, 1) * sizeof(T)) == cudaSuccess;
 }
 
+static bool recording(cudaStream_t st) {
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  if (!st || cudaStreamIsCapturing(st, &c) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return c == cudaStreamCaptureStatusActive;
+}
+
 static int path_prepare(Scene* s, const rq_path_params* p, PathParams& P, long long& total,
-                        int& chunk) {
+                        int& chunk, cudaStream_t st) {
   if (!p) return pfail(RQ_ERR_ARG, "NULL params");
   if (p->xres <= 0 || p->yres <= 0) return pfail(RQ_ERR_ARG, "bad resolution");
   const int strata = (int)std::lround(std::sqrt((double)p->spp));
@@ -123,7 +143,10 @@ static int path_prepare(Scene* s, const rq_path_params* p, PathParams& P, long l
   PathScratch* ps = s->paths;
   // 0: the whole frame, or equal parts of at most kAutoChunk paths - every
   // part pays the ends of its persistent stages again (two per bounce), where
-  // the SMs run out of paths.  Parts are made smaller while memory is short.
+  // the SMs run out of paths.  Parts are made smaller while memory is short, and
+  // fit the buffers that are there while the stream is recorded (nothing can be
+  // allocated then).
+  const bool rec = recording(st);
   long long parts = (total + kAutoChunk - 1) / kAutoChunk;
   for (;;) {
     long long ch = p->chunk_paths > 0 ? p->chunk_paths : (total + parts - 1) / parts;
@@ -131,6 +154,10 @@ static int path_prepare(Scene* s, const rq_path_params* p, PathParams& P, long l
     ch = std::max<long long>((p->chunk_paths > 0 ? ch : ch + p->spp - 1) / p->spp, 1) * p->spp;
     chunk = (int)std::min<long long>(ch, total);
     if (ps->capacity >= (size_t)chunk) break;
+    if (rec && p->chunk_paths <= 0 && ps->capacity >= (size_t)p->spp) {
+      parts = std::max(parts + 1, (total + (long long)ps->capacity - 1) / (long long)ps->capacity);
+      continue;
+    }
     if (ps->allocate((size_t)chunk)) break;
     cudaGetLastError();
     if (p->chunk_paths > 0 || chunk <= kLeastChunk)
@@ -150,6 +177,7 @@ static int path_prepare(Scene* s, const rq_path_params* p, PathParams& P, long l
     ps->host_materials.assign(mrgb, mrgb + 3 * p->n_materials);
   }
   P.materials = ps->materials;
+  ps->recorded = ps->recorded || rec;
   return RQ_OK;
 }
 
@@ -201,7 +229,7 @@ int rq_render_path_device(rq_scene* scene, const rq_path_params* params, float* 
   rq::PathParams P;
   long long total;
   int chunk;
-  int rc = rq::path_prepare(s, params, P, total, chunk);
+  int rc = rq::path_prepare(s, params, P, total, chunk, static_cast<cudaStream_t>(stream));
   if (rc != RQ_OK) return rc;
   return rq::path_run(s, P, total, chunk, d_rgb,
                       reinterpret_cast<unsigned long long*>(d_ray_counts),
@@ -217,7 +245,7 @@ int rq_render_path(rq_scene* scene, const rq_path_params* params, float* rgb,
   rq::PathParams P;
   long long total;
   int chunk;
-  int rc = rq::path_prepare(s, params, P, total, chunk);
+  int rc = rq::path_prepare(s, params, P, total, chunk, nullptr);
   if (rc != RQ_OK) return rc;
   rq::PathScratch* ps = s->paths;
   const size_t npix = (size_t)params->xres * params->yres;
