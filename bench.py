@@ -236,10 +236,10 @@ class PathFrame:
     # launches (bounces 0-3) of one full-size frame of this workload
     # (1280x720x16, 26.5M extension rays), summed over the launches and
     # divided by their rays.
-    DRAM_BYTES_PER_RAY = 65.7
+    DRAM_BYTES_PER_RAY = 72.9
     DRAM_BASIS = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the 4 "
-                  "path_extend_persistent_kernel launches of one full-size frame (1.744 GB "
-                  "over 26,534,621 extension rays = 65.7 B per ray) x extension rays per "
+                  "path_extend_persistent_kernel launches of one full-size frame (1.934 GB "
+                  "over 26,534,621 extension rays = 72.9 B per ray) x extension rays per "
                   "launch (all bounces / depth)")
 
     def traffic(self, rays):
@@ -250,17 +250,18 @@ class PathFrame:
     def launches_of(self, stage):
         return self.sc.max_depth
 
-    # What bounds the extension kernel, from one `ncu --set full` capture of
-    # bounce 0 at 640x360x4 spp (same scene): lanes active per warp
+    # What bounds the extension kernel, from the ncu counters of bounce 0
+    # at 640x360x4 spp (same scene): lanes active per warp
     # instruction, warps active vs the occupancy limit, issue-slot use,
     # L1/TEX and L2 throughput, long-scoreboard stalls per issued
     # instruction.
-    LIMITER = {"limiter": "dependent-load latency and SIMT efficiency, not HBM bandwidth",
-               "lanes_per_warp_instruction": 15.2, "warps_active_pct": 35.0,
-               "warps_active_theoretical_pct": 56.0, "issue_active_pct": 52.0,
-               "l1tex_throughput_pct": 40.5, "l2_throughput_pct": 6.2,
-               "long_scoreboard_stalls_per_issue": 5.71,
-               "profile": "profiles/path_extend_persistent_kernel_path_frame.md"}
+    LIMITER = {"limiter": "issue slots at half-full warps and dependent-load latency, "
+                          "not HBM bandwidth",
+               "lanes_per_warp_instruction": 16.8, "warps_active_pct": 38.4,
+               "warps_active_theoretical_pct": 50.0, "issue_active_pct": 58.0,
+               "l1tex_throughput_pct": 54.6, "l2_throughput_pct": 8.5,
+               "long_scoreboard_stalls_per_issue": 5.49,
+               "profile": "profiles/wide_walk_kernels.md"}
 
     def limiter(self):
         return dict(self.LIMITER)
@@ -429,9 +430,8 @@ class SmallFrame:
                 shadow * (32 + 4 + 32 * b_s + 48 * t_s),), per_ray
 
     # DRAM bytes per pixel of whitted_fused_kernel, from one ncu capture of
-    # this workload at full size (262,144 pixels: 4.84 MB read, 0.02 MB
-    # written).
-    DRAM_BYTES_PER_PIXEL = 18.6
+    # this workload at full size (262,144 pixels: 6.98 MB read).
+    DRAM_BYTES_PER_PIXEL = 26.6
 
     def traffic(self, rays):
         prim, _ = rays
@@ -630,12 +630,12 @@ class CoherentFrame:
 
     # DRAM bytes per primary ray of frame_primary_kernel, from one ncu
     # capture of this workload at 960x540 x 1 spp (518,400 rays, same scene).
-    DRAM_BYTES_PER_RAY = 127.7
+    DRAM_BYTES_PER_RAY = 182.0
 
     def traffic(self, rays):
         prim, _ = rays
         return self.DRAM_BYTES_PER_RAY * prim, ("ncu DRAM bytes per primary ray at 960x540x1 "
-                                                "(127.7 B) x primary rays of the launch")
+                                                "(182.0 B) x primary rays of the launch")
 
     def group_stages(self, stage_ms):
         return self.stage_names, [stage_ms[0], stage_ms[1], stage_ms[2]]
@@ -775,20 +775,19 @@ class BatchedQueriesWL:
 
     # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per ray of
     # batch_kernel: one ncu capture of the same 64 batches scaled by 1/4
-    # (7,080,009 rays; 1,275.7 MB read, 75.7 MB written) with the autotuned
-    # kind of configuration (split stack, 8 shared entries), scaled to a
-    # full launch by its rays (the batches and scenes are the same, so the
-    # re-read pattern per ray carries over).
-    DRAM_BYTES_PER_RAY = 190.9
+    # (7,080,009 rays; 1,690.9 MB read, 62.8 MB written) with the autotuned
+    # kind of configuration (wide walk), scaled to a full launch by its rays
+    # (the batches and scenes are the same, so the re-read pattern per ray
+    # carries over).
+    DRAM_BYTES_PER_RAY = 247.7
 
-    # What bounds batch_kernel, from one `ncu --set full` capture at 1/4 of
-    # the batch sizes (split stack, 8 shared entries, 48 registers).
-    LIMITER = {"limiter": "dependent-load latency and SIMT efficiency on uniformly random rays, "
+    # What bounds batch_kernel, from the ncu counters of that launch.
+    LIMITER = {"limiter": "L1 wavefronts and load latency of uniformly random rays, "
                           "not HBM bandwidth",
-               "lanes_per_warp_instruction": 8.67, "warps_active_pct": 55.2,
-               "warps_active_theoretical_pct": 62.5, "issue_active_pct": 61.5,
-               "long_scoreboard_stalls_per_issue": 7.88, "l1_hit_pct": 60.3,
-               "l2_hit_pct": 61.4}
+               "lanes_per_warp_instruction": 15.69, "warps_active_pct": 34.6,
+               "warps_active_theoretical_pct": 37.5, "issue_active_pct": 42.0,
+               "long_scoreboard_stalls_per_issue": 8.46, "l1tex_throughput_pct": 64.4,
+               "l1_hit_pct": 28.8, "l2_hit_pct": 53.0}
 
     def limiter(self):
         return dict(self.LIMITER)

@@ -1,5 +1,6 @@
-// Ray-query traversal kernels: closest hit and any hit over the paired-child
-// node records, Wald or Kensler-Shirley triangles.
+// Ray-query traversal kernels: closest hit and any hit over the four-wide
+// nodes, or over the paired-child node records (trees without wide nodes,
+// statistics), Wald or Kensler-Shirley triangles.
 //
 // Visit order follows DynBVH::intersectNode (Model/Groups/DynBVH.cc:274-404):
 // the child on the near side of the node's split axis first for closest
@@ -14,9 +15,8 @@
 //   * persistent: a grid sized to fill the GPU once, each warp fetching new
 //     rays with one atomicAdd per refill when `refill` or more of its lanes
 //     are idle (warp-ballot work stealing).
-// The traversal stack lives in shared memory, one column per thread
-// (stack[slot * blockDim + tid]), sized to the tree's depth so it can never
-// overflow.
+// The traversal stack lives in shared memory, one column per thread, sized to
+// the tree's depth so it can never overflow.
 #include <cuda_runtime.h>
 
 #include "rq_wide.cuh"

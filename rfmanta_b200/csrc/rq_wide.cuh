@@ -37,9 +37,9 @@
 // visits, reads a node in three loads for a record's four, and votes: a warp
 // stops descending once enough lanes wait at leaves, so leaves are tested by
 // more lanes together.  Measured against the binary walk: 777,777 camera rays
-// 246 -> 144 us, 2^20 random closest hits 234 -> 195 us, 3 M random occlusion
-// rays 578 -> 415 us, the 1280x720x16 path frame 11.38 -> 9.19 ms, the 512x512
-// Whitted frame 224 -> 138 us.  Eight-wide nodes would save a third more
+// 241 -> 136 us, 2^20 random closest hits 243 -> 199 us, 3 M random occlusion
+// rays 583 -> 399 us, the 512x512 Whitted frame 214 -> 128 us, the 1280x720x16
+// path frame 11.38 -> 8.68 ms (7.31 in one pass, rq_pathhost.cu).  Eight-wide nodes would save a third more
 // visits but cost as many instructions a ray (more order to keep) and more L1
 // wavefronts; 8-bit boxes halve the bytes but need twice the padding.
 //
