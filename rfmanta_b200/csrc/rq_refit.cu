@@ -166,7 +166,7 @@ int update_tree(Scene* s, int mode) {
     e = cudaGetLastError();
   }
   if (e == cudaSuccess)
-    e = s->make_wide(s->n_records, nullptr, reinterpret_cast<int*>(s->d_root_box + 6));
+    e = s->make_wide(s->n_records, s->n_leaf_tris, reinterpret_cast<int*>(s->d_root_box + 6));
   float root[7];
   if (e == cudaSuccess)
     e = cudaMemcpy(root, s->d_root_box, sizeof(root), cudaMemcpyDeviceToHost);

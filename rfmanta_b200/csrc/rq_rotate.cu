@@ -910,7 +910,7 @@ __global__ void emit_kernel(DynView V, const int32_t* __restrict__ tpos, int m_o
                             int32_t* perm, int n_objs, int32_t* rec_node, int32_t* rec_depth,
                             int32_t* rec_size) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m_max) return;
+  if (i >= m_max || st->error == 1) return;  // (1: the re-splits did not fit, paths are unknown)
   const int p = tree_position(i, tpos, m_old, nf_old, st);
   if (p < 0) return;
   int rec = 0, off = 0, dep = 0;
@@ -1165,7 +1165,8 @@ int rotate_update(Scene* s) {
   DY_CUDA(cudaGetLastError(), "relayout");
   DY_CUDA(launch_tri_setup(s->tri_kind, s->d_verts, s->d_idx, s->d_perm, N, s->d_tris, 0),
           "triangle records");
-  DY_CUDA(s->make_wide(s->rec_capacity, &d.st->n_records, &d.st->wide_bad), "wide nodes");
+  DY_CUDA(s->make_wide(s->rec_capacity, N, &d.st->wide_bad, &d.st->n_records, &d.st->error),
+          "wide nodes");
   UpdState out;
   DY_CUDA(cudaMemcpy(&out, d.st, sizeof(out), cudaMemcpyDeviceToHost), "update state");
   if (out.error != 0) {

@@ -273,7 +273,7 @@ int Scene::set_tree(const HostTree& t) {
     e = cudaMemcpy(d_level_recs, by_level.data(), nrec * sizeof(int32_t), cudaMemcpyHostToDevice);
   int bad = 1;
   if (e == cudaSuccess) e = cudaMemset(d_bad, 0, sizeof(int));
-  if (e == cudaSuccess) e = make_wide(nrec, nullptr, d_bad);
+  if (e == cudaSuccess) e = make_wide(nrec, (int)perm.size(), d_bad);
   if (e == cudaSuccess) e = cudaMemcpy(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return cuda_fail(e, "triangle setup");
   wide_ok = nrec > 0 && bad == 0;

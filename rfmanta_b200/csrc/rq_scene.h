@@ -187,7 +187,8 @@ struct Scene {
   float4* d_leaf_box = nullptr;
   bool wide_ok = false;
   float wide_extent = 0.f;
-  cudaError_t make_wide(int n, const int* n_dev, int* d_bad);
+  cudaError_t make_wide(int n, int n_tris, int* d_bad, const int* n_dev = nullptr,
+                        const int* error = nullptr);
   // d_nodes' allocation for `cap` records and their wide nodes
   static size_t record_bytes(int cap) { return wide_offset(cap) + (size_t)cap * 96; }
   static size_t wide_offset(int cap) { return ((size_t)cap * 64 + 255) / 256 * 256; }

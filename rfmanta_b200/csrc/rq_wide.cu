@@ -19,7 +19,9 @@
 // child, isLeftCheaper, in front).
 //
 // The thread also stores the boxes of r's leaf children (leaf_box) and
-// checks what the walk relies on: finite, nested boxes.
+// checks what the walk relies on: finite, nested boxes.  After an update that
+// failed on the device nothing is made, and a ref outside the tree is not
+// followed: records that a failed update never wrote hold anything.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -54,10 +56,15 @@ __device__ __forceinline__ uint32_t pair_bits(__half a, __half b) {
 }
 
 __global__ void __launch_bounds__(128)
-    wide_nodes_kernel(const float4* __restrict__ recs, int n, const int* n_dev, uint32_t* wide,
-                      float4* leaf_box, int* bad) {
+    wide_nodes_kernel(const float4* __restrict__ recs, int n, const int* n_dev, const int* error,
+                      int n_tris, uint32_t* wide, float4* leaf_box, int* bad) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= (n_dev ? min(n, *n_dev) : n)) return;
+  if (n_dev) n = min(n, *n_dev);
+  if (r >= n) return;
+  if (error && *error != 0) {
+    *bad = 1;
+    return;
+  }
   // largest coordinate of the scene, for the smallest cube
   RecBox rl, rr;
   record_boxes(recs, rl, rr);
@@ -100,7 +107,9 @@ __global__ void __launch_bounds__(128)
     const bool is_left = (k == 0) == left;
     const int c = is_left ? q3.x : q3.y;
     const RecBox b = side[is_left ? 0 : 1];
-    if (c < 0) {
+    if (c < 0 ? ~c >= n_tris : c >= n) {
+      ok = false;
+    } else if (c < 0) {
       ref[2 * k] = c;
       box[2 * k] = b;
       leaf_box[2 * (size_t)(~c)] = make_float4(b.lo[0], b.lo[1], b.lo[2], b.hi[0]);
@@ -157,11 +166,13 @@ __global__ void __launch_bounds__(128)
 }  // namespace
 
 // Launches the kernel over the scene's first n records, or the first
-// min(n, *n_dev) (on the legacy stream, where trees are made); *d_bad is set
-// to 1 where the tree cannot be walked wide.
-cudaError_t Scene::make_wide(int n, const int* n_dev, int* d_bad) {
+// min(n, *n_dev) of an update whose *error is 0 (on the legacy stream, where
+// trees are made), with n_tris triangles in their leaves; *d_bad is set to 1
+// where the tree cannot be walked wide.
+cudaError_t Scene::make_wide(int n, int n_tris, int* d_bad, const int* n_dev, const int* error) {
   if (n <= 0) return cudaSuccess;
-  wide_nodes_kernel<<<(n + 127) / 128, 128>>>(d_nodes, n, n_dev, d_wide, d_leaf_box, d_bad);
+  wide_nodes_kernel<<<(n + 127) / 128, 128>>>(d_nodes, n, n_dev, error, n_tris, d_wide,
+                                              d_leaf_box, d_bad);
   return cudaGetLastError();
 }
 
