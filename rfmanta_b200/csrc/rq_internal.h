@@ -58,6 +58,9 @@ int flag_compaction_tiles(int n);
 cudaError_t launch_flag_compaction(const uint8_t* flags, int n, int* tile_counts, int* total_out,
                                    int* qout, cudaStream_t st);
 
+// cudaMalloc, with rq_fail_allocation's failures.
+cudaError_t device_alloc(void** p, size_t bytes);
+
 void set_error(const std::string& msg);
 
 }  // namespace rq

@@ -149,6 +149,8 @@ namespace {
 // The update after the new positions are in the scene's device vertices.
 int update_tree(Scene* s, int mode) {
   if (mode == RQ_UPDATE_ROTATE) return rotate_update(s);
+  s->wide_ok = false;
+  ++s->generation;
   cudaError_t e = launch_tri_setup(s->tri_kind, s->d_verts, s->d_idx, s->d_perm,
                                    s->n_leaf_tris, s->d_tris, 0);
   const int nlev = (int)s->level_offsets.size() - 1;

@@ -974,6 +974,7 @@ int fail(int code, const std::string& msg) {
 }
 
 int cuda_fail(cudaError_t e, const char* what) {
+  cudaGetLastError();  // (a failed allocation is not the next launch's error)
   set_error(std::string("rotating update: ") + what + ": " + cudaGetErrorString(e));
   return e == cudaErrorMemoryAllocation ? RQ_ERR_OOM : RQ_ERR_CUDA;
 }
@@ -981,7 +982,7 @@ int cuda_fail(cudaError_t e, const char* what) {
 template <typename T>
 cudaError_t dalloc(DynTree* d, T** p, size_t count) {
   void* q = nullptr;
-  const cudaError_t e = cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T));
+  const cudaError_t e = device_alloc(&q, std::max<size_t>(count, 1) * sizeof(T));
   if (e == cudaSuccess) {
     d->allocs.push_back(q);
     *p = static_cast<T*>(q);
@@ -995,14 +996,21 @@ cudaError_t dalloc(DynTree* d, T** p, size_t count) {
     if (e_ != cudaSuccess) return cuda_fail(e_, what); \
   } while (0)
 
-// Grows the record buffers to hold any tree over the scene's objects.
+// Grows the record buffers to hold any tree over the scene's objects; what
+// the buffers hold goes with it, so the scene can be used as before whatever
+// the rest of the update does.
 int ensure_record_capacity(Scene* s) {
   const int need = std::max(s->n_tris - 1, 1);
   if (s->rec_capacity >= need) return RQ_OK;
-  float4* nodes = nullptr;
-  int32_t* levels = nullptr;
-  DY_CUDA(cudaMalloc(&nodes, Scene::record_bytes(need)), "record buffer");
-  cudaError_t e = cudaMalloc(&levels, (size_t)need * sizeof(int32_t));
+  void *nodes_mem = nullptr, *levels_mem = nullptr;
+  DY_CUDA(device_alloc(&nodes_mem, Scene::record_bytes(need)), "record buffer");
+  cudaError_t e = device_alloc(&levels_mem, (size_t)need * sizeof(int32_t));
+  float4* nodes = static_cast<float4*>(nodes_mem);
+  int32_t* levels = static_cast<int32_t*>(levels_mem);
+  uint32_t* wide = reinterpret_cast<uint32_t*>(static_cast<char*>(nodes_mem) +
+                                               Scene::wide_offset(need));
+  if (e == cudaSuccess && s->n_records > 0)
+    e = cudaMemcpy(wide, s->d_wide, (size_t)s->n_records * 96, cudaMemcpyDeviceToDevice);
   if (e == cudaSuccess && s->n_records > 0)
     e = cudaMemcpy(nodes, s->d_nodes, (size_t)s->n_records * 4 * sizeof(float4),
                    cudaMemcpyDeviceToDevice);
@@ -1017,10 +1025,10 @@ int ensure_record_capacity(Scene* s) {
   cudaFree(s->d_nodes);
   cudaFree(s->d_level_recs);
   s->d_nodes = nodes;
-  s->d_wide = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(nodes) +
-                                          Scene::wide_offset(need));
+  s->d_wide = wide;
   s->d_level_recs = levels;
   s->rec_capacity = need;
+  ++s->generation;
   return RQ_OK;
 }
 
@@ -1126,6 +1134,8 @@ int rotate_update(Scene* s) {
                 "the rotating update needs a tree whose leaves hold every triangle once");
   int rc = dyn_sync(s);
   if (rc != RQ_OK) return rc;
+  s->wide_ok = false;
+  ++s->generation;
   DynTree& d = *s->dyn;
   const DynView V = view(d);
   const int N = s->n_tris;

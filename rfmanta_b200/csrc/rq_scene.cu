@@ -30,6 +30,13 @@ static thread_local std::string g_error;
 
 void set_error(const std::string& msg) { g_error = msg; }
 
+static thread_local int g_fail_allocation = 0;  // this one from now on fails, 0: none
+
+cudaError_t device_alloc(void** p, size_t bytes) {
+  if (g_fail_allocation > 0 && --g_fail_allocation == 0) return cudaErrorMemoryAllocation;
+  return cudaMalloc(p, bytes);
+}
+
 static int fail(int code, const std::string& msg) {
   set_error(msg);
   return code;
@@ -458,6 +465,12 @@ using rq::cuda_fail;
 extern "C" {
 
 const char* rq_last_error(void) { return rq::g_error.c_str(); }
+
+int rq_fail_allocation(int nth) {
+  if (nth < 0) return fail(RQ_ERR_ARG, "nth must be >= 0");
+  rq::g_fail_allocation = nth;
+  return RQ_OK;
+}
 
 const char* rq_version(void) { return "rfmanta_b200 0.1.0 sm_100a"; }
 

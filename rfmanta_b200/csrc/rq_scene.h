@@ -181,8 +181,9 @@ struct Scene {
   // four-wide nodes of the tree (rq_wide.cu), one per record, behind the
   // records in d_nodes' allocation, and the leaves' boxes, behind the triangle
   // records in d_tris': made with the tree and after every update.  wide_ok =
-  // the tree can be walked wide; wide_extent = largest coordinate of the root
-  // record's boxes
+  // the tree can be walked wide (false while an update changes the records, so
+  // one that stops half way leaves the walk over them); wide_extent = largest
+  // coordinate of the root record's boxes
   uint32_t* d_wide = nullptr;
   float4* d_leaf_box = nullptr;
   bool wide_ok = false;

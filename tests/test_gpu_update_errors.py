@@ -107,3 +107,46 @@ def test_an_update_that_grows_too_deep_is_an_error_and_no_more():
     assert _hits(b).hitPrim.shape == want.hitPrim.shape
     b.close()
     other.close()
+
+
+@pytest.mark.gpu
+def test_an_update_out_of_memory_leaves_the_scene_as_it_was():
+    """Every device allocation of the first rotating update fails in turn:
+    the record buffers have moved by then, and the scene and a plan made
+    before it give the answers they gave."""
+    import torch
+    from rfmanta_b200 import _lib, scenes
+    from rfmanta_b200.batch import BatchedQueries, QueryBatch
+    b = _sphere()
+    o, d, _, _ = scenes.random_rays(4096, np.full(3, -2.0), np.full(3, 2.0), seed=5,
+                                    anyhit_fraction=0.0)
+    q = QueryBatch(0, *(torch.from_numpy(x).cuda() for x in (o, d)),
+                   torch.full((o.shape[1],), 1e19, device="cuda"))
+    plan = BatchedQueries([b], [q])
+
+    def answers():
+        plan.launch()
+        torch.cuda.synchronize()
+        r = _hits(b)
+        return [plan.t[0].cpu().numpy(), plan.prim[0].cpu().numpy(), r.minT, r.hitPrim]
+
+    want = answers()
+    failed = 0
+    for nth in range(1, 64):
+        _lib.check(_lib.lib.rq_fail_allocation(nth))
+        try:
+            b.update(rotate=True)
+        except _lib.RQError as e:
+            assert e.code == _lib.RQ_ERR_OOM
+            failed += 1
+        else:
+            break
+        finally:
+            _lib.lib.rq_fail_allocation(0)
+        for got, w in zip(answers(), want):
+            assert np.array_equal(got, w)
+    assert 10 < failed < 63
+    got = answers()  # (the update moved no vertex: the same hits from the rotated tree)
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[2], want[2])
+    plan.close()
+    b.close()
