@@ -115,6 +115,7 @@ void Scene::free_tree() {
   tree_from_dyn = false;
   tree_stale = false;
   has_tree = false;
+  ++generation;  // plans and servers hold this tree's pointers
 }
 
 DevScene Scene::dev() const {
@@ -243,12 +244,12 @@ int Scene::set_tree(const HostTree& t) {
   free_tree();
   const int nrec = L.n_records;
   const int cap = std::max(nrec, 1);
-  RQ_CUDA(cudaMalloc(&d_nodes, record_bytes(cap)));
+  RQ_CUDA(device_alloc(reinterpret_cast<void**>(&d_nodes), record_bytes(cap)));
   d_wide = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(d_nodes) + wide_offset(cap));
   // one allocation: triangle records, leaf boxes, leaf order, a flag
   const size_t np = std::max<size_t>(perm.size(), 1);
   const size_t box_off = (np * 48 + 255) / 256 * 256, perm_off = box_off + np * 32;
-  RQ_CUDA(cudaMalloc(&d_tris, perm_off + (np + 1) * 4));
+  RQ_CUDA(device_alloc(reinterpret_cast<void**>(&d_tris), perm_off + (np + 1) * 4));
   char* tri_mem = reinterpret_cast<char*>(d_tris);
   d_leaf_box = reinterpret_cast<float4*>(tri_mem + box_off);
   d_perm = reinterpret_cast<int32_t*>(tri_mem + perm_off);
@@ -275,7 +276,8 @@ int Scene::set_tree(const HostTree& t) {
     for (int r = 0; r < nrec; ++r) by_level[fill[maxd - L.rec_depth[r]]++] = r;
     level_offsets.assign(start.begin(), start.end());
   }
-  if (e == cudaSuccess) e = cudaMalloc(&d_level_recs, std::max(nrec, 1) * sizeof(int32_t));
+  if (e == cudaSuccess)
+    e = device_alloc(reinterpret_cast<void**>(&d_level_recs), std::max(nrec, 1) * sizeof(int32_t));
   if (e == cudaSuccess && nrec > 0)
     e = cudaMemcpy(d_level_recs, by_level.data(), nrec * sizeof(int32_t), cudaMemcpyHostToDevice);
   int bad = 1;

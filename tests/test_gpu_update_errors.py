@@ -150,3 +150,36 @@ def test_an_update_out_of_memory_leaves_the_scene_as_it_was():
     assert np.array_equal(got[0], want[0]) and np.array_equal(got[2], want[2])
     plan.close()
     b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nth", [1, 2, 3])
+def test_a_plan_refuses_a_scene_that_lost_its_tree(nth):
+    """An import out of memory has freed the old tree, which the plan's table
+    still points at."""
+    import torch
+    from rfmanta_b200 import _lib
+    from rfmanta_b200.batch import BatchedQueries, QueryBatch
+    b = _sphere()
+    blob = b.exportBlob()
+    n = 64
+    q = QueryBatch(0, torch.zeros(3, n, device="cuda"), torch.ones(3, n, device="cuda"),
+                   torch.ones(n, device="cuda"))
+    plan = BatchedQueries([b], [q])
+    plan.launch()
+    torch.cuda.synchronize()
+    _lib.check(_lib.lib.rq_fail_allocation(nth))
+    try:
+        with pytest.raises(_lib.RQError) as e:
+            b.importBlob(blob)
+        assert e.value.code == _lib.RQ_ERR_OOM
+    finally:
+        _lib.lib.rq_fail_allocation(0)
+    with pytest.raises(_lib.RQError) as e:
+        plan.launch()
+    assert e.value.code == _lib.RQ_ERR_STATE
+    b.importBlob(blob)
+    plan.launch()
+    torch.cuda.synchronize()
+    plan.close()
+    b.close()
