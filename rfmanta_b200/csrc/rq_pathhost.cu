@@ -38,6 +38,18 @@ struct PathScratch {
   // set per recorded size: capacities only grow).
   bool recorded = false;
   std::vector<void*> retired;
+  // The recorded kernels read the material table too; one they hold is kept
+  // in the same way when a frame brings other materials.
+  bool materials_recorded = false;
+  void free_materials() {
+    if (materials_recorded)
+      retired.push_back(materials);
+    else
+      cudaFree(materials);
+    materials = nullptr;
+    host_materials.clear();
+    materials_recorded = false;
+  }
   void free_paths() {
     if (recorded)
       retired.push_back(memory);
@@ -184,8 +196,7 @@ static int path_prepare(Scene* s, const rq_path_params* p, PathParams& P, long l
   const float* mrgb = p->material_rgb;
   if ((int)ps->host_materials.size() != 3 * p->n_materials ||
       std::memcmp(ps->host_materials.data(), mrgb, sizeof(float) * 3 * p->n_materials) != 0) {
-    cudaFree(ps->materials);
-    ps->materials = nullptr;
+    ps->free_materials();
     if (!palloc(&ps->materials, 3 * (size_t)p->n_materials) ||
         cudaMemcpy(ps->materials, mrgb, sizeof(float) * 3 * p->n_materials,
                    cudaMemcpyHostToDevice) != cudaSuccess)
@@ -194,6 +205,7 @@ static int path_prepare(Scene* s, const rq_path_params* p, PathParams& P, long l
   }
   P.materials = ps->materials;
   ps->recorded = ps->recorded || rec;
+  ps->materials_recorded = ps->materials_recorded || rec;
   return RQ_OK;
 }
 
