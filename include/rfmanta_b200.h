@@ -70,8 +70,8 @@ RQ_API const char* rq_version(void);
 
 /*
  * For tests of what callers see when memory is short: the nth device
- * allocation that this host thread's tree imports and updates make from now
- * on fails on the host (RQ_ERR_OOM); 0 takes the failure back.  Other threads
+ * allocation that this host thread's tree imports, updates and path frames
+ * make from now on fails on the host (RQ_ERR_OOM); 0 takes the failure back.  Other threads
  * and calls are not affected.
  */
 RQ_API int rq_fail_allocation(int nth);
@@ -699,7 +699,8 @@ typedef struct {
   const float* material_rgb;      /* host: n_materials x (r, g, b) */
   int chunk_paths;                /* paths per wavefront pass, 0 = the whole frame, or
                                      equal parts of at most 32Mi paths (77 bytes of
-                                     device memory each; smaller where that is short) */
+                                     device memory each, kept by the scene; above
+                                     4Mi paths at most an eighth of what is free) */
   rq_environment environment;     /* zero = constant ambient and background;
                                      EyeAmbient at the last bounce sees the
                                      direction sampled there, as the

@@ -15,11 +15,15 @@
 
 namespace rq {
 
-// Paths per wavefront pass when the caller leaves it to the library, and where
-// it stops trying smaller passes.  The 1280x720x16 frame in passes of 2 / 4 / 8 /
-// 16 Mi paths: 10.57 / 8.68 / 7.91 / 7.33 ms; 77 bytes of state per path.
+// Paths per wavefront pass when the caller leaves it to the library.  The
+// 1280x720x16 frame in passes of 2 / 4 / 8 / 16 Mi paths: 10.57 / 8.68 / 7.91 /
+// 7.33 ms; 77 bytes of state per path, kept by the scene.  Passes above
+// kPlainChunk (0.32 GB) take at most an eighth of the memory that is free, so
+// that other scenes, servers and the caller's own tensors find theirs.
 constexpr long long kAutoChunk = 32LL << 20;
-constexpr long long kLeastChunk = 1LL << 20;
+constexpr long long kPlainChunk = 4LL << 20;
+constexpr long long kLeastChunk = 1LL << 20;  // smaller passes are not tried
+constexpr long long kPathBytes = 77;
 
 struct PathScratch {
   size_t capacity = 0;
@@ -38,6 +42,9 @@ struct PathScratch {
   // set per recorded size: capacities only grow).
   bool recorded = false;
   std::vector<void*> retired;
+  // An allocation failed: frames fit their passes to the buffers there are
+  // instead of failing it again each time.
+  bool was_short = false;
   // The recorded kernels read the material table too; one they hold is kept
   // in the same way when a frame brings other materials.
   bool materials_recorded = false;
@@ -60,36 +67,47 @@ struct PathScratch {
     recorded = false;
     capacity = 0;
   }
-  bool allocate(size_t C) {
-    free_paths();
+  // Places B's buffers for C paths from `base` on; returns their bytes.
+  static size_t place(char* base, size_t C, PathBuffers& B) {
     size_t bytes = 0;
-    auto place = [&](auto*& q, size_t n) {
+    auto at = [&](auto*& q, size_t n) {
       using T = std::remove_reference_t<decltype(*q)>;
-      q = memory ? reinterpret_cast<T*>(static_cast<char*>(memory) + bytes) : nullptr;
+      q = base ? reinterpret_cast<T*>(base + bytes) : nullptr;
       bytes += (std::max<size_t>(n, 1) * sizeof(T) + 255) / 256 * 256;
     };
-    auto lay_out = [&] {
-      bytes = 0;
-      place(B.o, 3 * C);
-      place(B.d, 3 * C);
-      place(B.imp, 3 * C);
-      place(B.rad, 3 * C);
-      place(B.rng, C);
-      place(B.t, C);
-      place(B.pos, C);
-      place(B.prim, C);
-      place(B.queue[0], C);
-      place(B.queue[1], C);
-      place(B.counters, kPathCounters);
-      place(B.alive, C);
-      place(B.tile_counts, C / 4096 + 2);
-    };
-    lay_out();
-    if (cudaMalloc(&memory, bytes) != cudaSuccess) {
-      memory = nullptr;
+    at(B.o, 3 * C);
+    at(B.d, 3 * C);
+    at(B.imp, 3 * C);
+    at(B.rad, 3 * C);
+    at(B.rng, C);
+    at(B.t, C);
+    at(B.pos, C);
+    at(B.prim, C);
+    at(B.queue[0], C);
+    at(B.queue[1], C);
+    at(B.counters, kPathCounters);
+    at(B.alive, C);
+    at(B.tile_counts, C / 4096 + 2);
+    return bytes;
+  }
+  // Buffers for C paths; the ones there are given up once the new ones are
+  // there, or before, where only one set fits.
+  bool allocate(size_t C) {
+    PathBuffers none{};
+    const size_t bytes = place(nullptr, C, none);
+    void* fresh = nullptr;
+    cudaError_t e = device_alloc(&fresh, bytes);
+    if (e != cudaSuccess && memory && !recorded) {
+      free_paths();
+      e = device_alloc(&fresh, bytes);
+    }
+    if (e != cudaSuccess) {
+      cudaGetLastError();
       return false;
     }
-    lay_out();
+    free_paths();
+    memory = fresh;
+    place(static_cast<char*>(memory), C, B);
     capacity = C;
     B.capacity = C;
     return true;
@@ -172,24 +190,34 @@ static int path_prepare(Scene* s, const rq_path_params* p, PathParams& P, long l
   // 0: the whole frame, or equal parts of at most kAutoChunk paths - every
   // part pays the ends of its persistent stages again (two per bounce), where
   // the SMs run out of paths.  Parts are made smaller while memory is short, and
-  // fit the buffers that are there while the stream is recorded (nothing can be
-  // allocated then).
-  const bool rec = recording(st);
-  long long parts = (total + kAutoChunk - 1) / kAutoChunk;
+  // fit the buffers that are there where it has been short before and while the
+  // stream is recorded (nothing can be allocated then).  A debug dump is one
+  // pass, of at most kPlainChunk.
+  const bool rec = recording(st), own = p->chunk_paths > 0;
+  const auto in_parts = [&](long long parts) {  // whole pixels per chunk
+    const long long ch = own ? p->chunk_paths : (total + parts - 1) / parts + p->spp - 1;
+    return (int)std::min(std::max<long long>(ch / p->spp, 1) * p->spp, total);
+  };
+  const long long most = s->path_dbg_prim ? kPlainChunk : kAutoChunk;
+  long long parts = (total + most - 1) / most;
+  const bool fit = !own && ps->capacity >= (size_t)p->spp && (rec || ps->was_short);
+  if (!fit && !own && in_parts(parts) > std::max(kPlainChunk, (long long)ps->capacity)) {
+    size_t spare = 0, all = 0;
+    if (cudaMemGetInfo(&spare, &all) != cudaSuccess) cudaGetLastError();
+    const long long share = std::max({kPlainChunk, (long long)ps->capacity,
+                                      (long long)spare / 8 / kPathBytes});
+    parts = std::max(parts, (total + share - 1) / share);
+  }
   for (;;) {
-    long long ch = p->chunk_paths > 0 ? p->chunk_paths : (total + parts - 1) / parts;
-    // whole pixels per chunk
-    ch = std::max<long long>((p->chunk_paths > 0 ? ch : ch + p->spp - 1) / p->spp, 1) * p->spp;
-    chunk = (int)std::min<long long>(ch, total);
+    chunk = in_parts(parts);
     if (ps->capacity >= (size_t)chunk) break;
-    if (rec && p->chunk_paths <= 0 && ps->capacity >= (size_t)p->spp) {
+    if (fit) {
       parts = std::max(parts + 1, (total + (long long)ps->capacity - 1) / (long long)ps->capacity);
       continue;
     }
     if (ps->allocate((size_t)chunk)) break;
-    cudaGetLastError();
-    if (p->chunk_paths > 0 || chunk <= kLeastChunk)
-      return pfail(RQ_ERR_OOM, "path state allocation failed");
+    if (own || chunk <= kLeastChunk) return pfail(RQ_ERR_OOM, "path state allocation failed");
+    ps->was_short = true;
     parts *= 2;
   }
   if (!ps->counts && !palloc(&ps->counts, 2)) return pfail(RQ_ERR_OOM, "counter allocation");
