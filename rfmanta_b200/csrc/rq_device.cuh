@@ -213,7 +213,7 @@ struct DevScene {
   // four-wide nodes (rq_wide.cu), one per record; NULL: the tree has none
   const uint32_t* wide;
   const float4* leaf_box;  // 2 float4 per leaf, at its first triangle: lo xyz hi.x | hi.yz
-  float origin_limit;      // largest |origin| component the wide walk takes
+  float wide_lo[3], wide_hi[3];  // origins the wide walk takes
 };
 
 }  // namespace rq

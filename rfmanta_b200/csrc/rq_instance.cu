@@ -72,13 +72,12 @@ static size_t two_level_bytes(const Scene& s, int block, bool wide) {
 
 bool Scene::inner_wide() const {
   // rays reach an instance from anywhere in the scene and some way outside:
-  // the inner scenes' origin limits (kWideOrigin of their sizes) must cover
-  // four times the scene, or too many of them would take the exact walk
+  // the inner scenes' origin limits (kWideOrigin of their half sizes) must cover
+  // four half sizes of the scene, or too many of them would take the exact walk
   float size = 0.f;
-  for (int c = 0; c < 3; ++c)
-    size = std::max(size, std::max(std::fabs(root_lo[c]), std::fabs(root_hi[c])));
+  for (int c = 0; c < 3; ++c) size = std::max(size, 0.5f * root_hi[c] - 0.5f * root_lo[c]);
   for (const Scene* b : blas)
-    if (!b->dev().wide || kWideOrigin * b->wide_extent < 4.f * size) return false;
+    if (!b->dev().wide || b->wide_reach < 4.f * size) return false;
   return instanced;
 }
 

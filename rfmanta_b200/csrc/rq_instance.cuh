@@ -41,7 +41,7 @@ __device__ __forceinline__ void trace_two_level(const DevScene& T, const DevScen
   if (WIDE) {
     wst.init(reinterpret_cast<int*>(stk - threadIdx.x + (size_t)T.depth * stride) + threadIdx.x,
              stride);
-    wide_ok = wide_setup(INFINITY, r, ANY, w);  // (the origin is checked per instance)
+    wide_ok = wide_setup(r, ANY, w);
   }
   for (;;) {
     while (ref >= 0 && ref != kDone) {
@@ -97,9 +97,7 @@ __device__ __forceinline__ void trace_two_level(const DevScene& T, const DevScen
       if (STATS) cnt->boxes += 1;
       start_ray(S, lr, lh, lref, lsp);
       if (WIDE) {
-        const float lim = S.origin_limit;
-        if (lref != kDone && !(wide_ok && fabsf(lr.o[0]) <= lim && fabsf(lr.o[1]) <= lim &&
-                               fabsf(lr.o[2]) <= lim)) {
+        if (lref != kDone && !(wide_ok && wide_origin(S, lr.o))) {
           lh = wide_trace_exact<KIND, ANY>(S.nodes, S.tris, lref, lr);
           lr.minT = lh.id >= 0 ? lh.t : lr.minT;
           lref = kDone;

@@ -182,9 +182,7 @@ int update_tree(Scene* s, int mode) {
   }
   int wide_bad;
   std::memcpy(&wide_bad, &root[6], sizeof(int));
-  s->wide_ok = s->n_records > 0 && wide_bad == 0;
-  s->wide_extent = 0.f;
-  for (int k = 0; k < 6; ++k) s->wide_extent = std::max(s->wide_extent, std::fabs(root[k]));
+  s->set_wide(s->n_records > 0 && wide_bad == 0, root, root + 3);
   s->tree_stale = true;
   s->tree_from_dyn = false;
   if (s->dyn) mark_dyn_bounds_stale(s->dyn);

@@ -1191,9 +1191,7 @@ int rotate_update(Scene* s) {
   d.layout_host_stale = true;
   s->n_records = out.n_records;
   s->n_leaves = out.n_records + 1;
-  s->wide_ok = out.n_records > 0 && out.wide_bad == 0;
-  s->wide_extent = 0.f;
-  for (float x : out.root) s->wide_extent = std::max(s->wide_extent, std::fabs(x));
+  s->set_wide(out.n_records > 0 && out.wide_bad == 0, out.root, out.root + 3);
   s->root_ref = out.n_records > 0 ? 0 : ~0;
   for (int c = 0; c < 3; ++c) {
     s->root_lo[c] = out.root[c];

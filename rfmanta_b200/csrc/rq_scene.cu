@@ -132,8 +132,23 @@ DevScene Scene::dev() const {
   S.depth = depth > 0 ? depth : 1;
   S.wide = wide_ok && depth <= kWideMaxDepth ? d_wide : nullptr;
   S.leaf_box = d_leaf_box;
-  S.origin_limit = kWideOrigin * wide_extent;
+  for (int c = 0; c < 3; ++c) {
+    const float mid = 0.5f * wide_box[c] + 0.5f * wide_box[3 + c];
+    S.wide_lo[c] = mid - wide_reach;
+    S.wide_hi[c] = mid + wide_reach;
+  }
   return S;
+}
+
+void Scene::set_wide(bool ok, const float* lo, const float* hi) {
+  wide_ok = ok;
+  float half = 0.f;
+  for (int c = 0; c < 3; ++c) {
+    wide_box[c] = lo[c];
+    wide_box[3 + c] = hi[c];
+    half = std::max(half, 0.5f * hi[c] - 0.5f * lo[c]);
+  }
+  wide_reach = kWideOrigin * half;
 }
 
 // ---------------------------------------------------------------- tree ----
@@ -285,10 +300,15 @@ int Scene::set_tree(const HostTree& t) {
   if (e == cudaSuccess) e = make_wide(nrec, (int)perm.size(), d_bad);
   if (e == cudaSuccess) e = cudaMemcpy(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return cuda_fail(e, "triangle setup");
-  wide_ok = nrec > 0 && bad == 0;
-  wide_extent = 0.f;
-  for (int k = 0; wide_ok && k < 12; ++k)  // the root record's two boxes
-    wide_extent = std::max(wide_extent, std::fabs(reinterpret_cast<const float*>(recs.data())[k]));
+  if (nrec > 0) {  // the root record's two boxes (the imported root box may be any)
+    float lo[3], hi[3];
+    const float* q = reinterpret_cast<const float*>(recs.data());
+    for (int c = 0; c < 3; ++c) {
+      lo[c] = std::min(q[c], q[6 + c]);
+      hi[c] = std::max(q[3 + c], q[9 + c]);
+    }
+    set_wide(bad == 0, lo, hi);
+  }
   rec_node = L.rec_node;
   rec_depth = L.rec_depth;
   rec_size = L.rec_size;

@@ -182,12 +182,13 @@ struct Scene {
   // records in d_nodes' allocation, and the leaves' boxes, behind the triangle
   // records in d_tris': made with the tree and after every update.  wide_ok =
   // the tree can be walked wide (false while an update changes the records, so
-  // one that stops half way leaves the walk over them); wide_extent = largest
-  // coordinate of the root record's boxes
+  // one that stops half way leaves the walk over them); wide_box = the root
+  // record's boxes as one and wide_reach how far outside its centre origins lie
   uint32_t* d_wide = nullptr;
   float4* d_leaf_box = nullptr;
   bool wide_ok = false;
-  float wide_extent = 0.f;
+  float wide_box[6] = {}, wide_reach = 0.f;
+  void set_wide(bool ok, const float* lo, const float* hi);
   cudaError_t make_wide(int n, int n_tris, int* d_bad, const int* n_dev = nullptr,
                         const int* error = nullptr);
   // d_nodes' allocation for `cap` records and their wide nodes

@@ -91,7 +91,6 @@ __global__ void __launch_bounds__(128)
   }
   const float size = fmaxf(ext, big * kWideMinCube);
   const float gs = __frcp_rn(size);
-  const float pad = kWidePad + kWidePad32 * (kWideOrigin + 1.f) * big * gs * 1.001f;
   float pb[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) pb[c] = (0.5f * lo[c] + 0.5f * hi[c]) * gs;
@@ -148,7 +147,7 @@ __global__ void __launch_bounds__(128)
       const double a = (double)box[k].lo[c] * gs - pb[c], b = (double)box[k].hi[c] * gs - pb[c];
       ce[k] = __float2half((float)(0.5 * (a + b)));
       const double m = (double)__half2float(ce[k]);
-      he[k] = __float2half_ru(__double2float_ru(fmax(b - m, m - a) + (double)pad));
+      he[k] = __float2half_ru(__double2float_ru(fmax(b - m, m - a) + (double)kWidePad));
     }
     w[8 + 2 * c] = pair_bits(ce[0], ce[1]);
     w[9 + 2 * c] = pair_bits(ce[2], ce[3]);

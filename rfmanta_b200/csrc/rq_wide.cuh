@@ -20,16 +20,21 @@
 //     whose exact box is hit was hit too, with a minT at least as large: the
 //     leaf's own test stands for the whole chain.
 //
-// Error bound.  In units of the node's cube (half size at most 0.57 with its
-// padding), with u = 2^-11 (half rounding), the reference point is the ray's
-// closest point to the cube's centre, within 0.98 of it when the ray meets the
-// cube, so a plane lies within 1.5 of it.  A plane's time carries errors of
-// 0.98 u (offset) + 0.5 u (slope) + 1.5 u (centre) + 0.53 u (extent) + 1.5 u
-// (sum) < 2.5e-3 = kWidePad, and those of the 32-bit origin and slope and of
-// the exact test's own rounding, 7 * 2^-24 of the distance to the origin, which
-// is below (kWideOrigin + 1) scene sizes: kWidePad32 of that is added, in the
-// scene's units (and bounds the smallest cube).  Times against minT carry a
-// slack of 2^-8 cubes and 2^-22 of the distance.
+// Error bound.  In units of the node's cube (boxes within 0.565 of its centre,
+// padding included) the reference point is the ray's closest point to the
+// cube's centre.  A ray that meets the cube has it within 0.98, and within 0.78
+// along one axis, so a plane lies within 1.34 of it.  With u = 2^-11 (half
+// rounding), a plane's time carries errors, as positions along its axis, of
+// 0.78 u (offset) + 0.5 u (slope) + 1.34 u (centre) + 0.53 u (extent) + 1.34 u
+// (sum) = 4.5 u = 2.2e-3 < kWidePad, by which the node's boxes are larger.
+// The 32-bit roundings - the origin in cube units (one multiply-add, so relative
+// to the distance, not to the coordinate: the boxes are placed in double around
+// the rounded centre), the slope, and two of the exact test - are 4 * 2^-24 of
+// the time to the plane, at most 7 against a bound (minT); both planes of a
+// comparison together, 8 * 2^-24 of the time to the cube: kWide32 of it is added
+// to every exit time.  So the padding grows with the ray's own distance and
+// costs nothing near by, wherever the scene lies and however fine it is.  Times
+// against 0 and minT carry 2^-8 cubes more.
 //
 // What it is for: the binary walk is bound by issue slots (52-57% issued, 10-15
 // of 32 lanes) and by the dependent record loads (13 to 31 visits a ray), and on
@@ -44,7 +49,8 @@
 // wavefronts; 8-bit boxes halve the bytes but need twice the padding.
 //
 // Rays outside these bounds (an infinite inverse direction, a slope above
-// kWideSlope, an origin farther than kWideOrigin scene sizes) take the exact
+// kWideSlope, an origin more than kWideOrigin half sizes from the scene's centre)
+// take the exact
 // binary walk with a stack in local memory (wide_trace_exact).
 #pragma once
 
@@ -55,11 +61,14 @@
 namespace rq {
 
 constexpr float kWidePad = 2.5e-3f;
-constexpr float kWidePad32 = 4.8e-7f;   // 8 * 2^-24
+constexpr float kWide32 = 5e-7f;        // 8.4 * 2^-24
 constexpr float kWideSlope = 16384.f;   // largest |d|max / |d_k|
-constexpr float kWideOrigin = 64.f;     // largest |origin| over the scene's largest |coordinate|
-// cubes are at least 16 times the 32-bit padding
-constexpr float kWideMinCube = 16.f * kWidePad32 * (kWideOrigin + 1.f);
+// Distance of an origin from the scene's centre in (largest) half sizes.  The
+// bound above needs kWideOrigin / kWideMinCube * kWide32 to stay a half number.
+constexpr float kWideOrigin = 64.f;
+// Smallest cube over the scene's largest |coordinate|: 32 roundings of it, so
+// that the rounded centre is within 2/32 of the box's.
+constexpr float kWideMinCube = 1.f / (1 << 19);
 constexpr int kWideMaxDepth = 64;       // binary depth the local-memory stack takes
 
 // What a wide visit needs of a ray beside the Ray itself.
@@ -74,10 +83,8 @@ struct WideRay {
                       // (closest hit); all set: any hit
 };
 
-// Prepares a ray; false when it must take the exact walk in a tree with this
-// origin limit.
-__device__ __forceinline__ bool wide_setup(float origin_limit, const Ray& r, bool any,
-                                           WideRay& w) {
+// Prepares a ray but for its origin; false when it must take the exact walk.
+__device__ __forceinline__ bool wide_setup(const Ray& r, bool any, WideRay& w) {
   const float ax = fabsf(r.d[0]), ay = fabsf(r.d[1]), az = fabsf(r.d[2]);
   w.dm = fmaxf(fmaxf(ax, ay), az);
   bool ok = w.dm > 1e-15f && w.dm < 1e15f && !(r.minT != r.minT);
@@ -86,7 +93,7 @@ __device__ __forceinline__ bool wide_setup(float origin_limit, const Ray& r, boo
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     w.A[c] = w.dm * r.inv[c];
-    ok = ok && fabsf(w.A[c]) <= kWideSlope && fabsf(r.o[c]) <= origin_limit;
+    ok = ok && fabsf(w.A[c]) <= kWideSlope;
     g[c] = r.d[c] * rd;
     sum = __fmaf_rn(g[c], g[c], sum);
     w.a2[c] = __float2half2_rn(w.A[c]);
@@ -99,6 +106,14 @@ __device__ __forceinline__ bool wide_setup(float origin_limit, const Ray& r, boo
   const unsigned up =
       (r.d[0] > 0.f ? 1u : 0u) | (r.d[1] > 0.f ? 2u : 0u) | (r.d[2] > 0.f ? 4u : 0u);
   w.side = 0x010101u * (any ? 0x3fu : up | (~up & 7u) << 3);
+  return ok;
+}
+
+// Whether a tree takes rays from this origin over its wide nodes.
+__device__ __forceinline__ bool wide_origin(const DevScene& S, const float* o) {
+  bool ok = true;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) ok = ok && o[c] >= S.wide_lo[c] && o[c] <= S.wide_hi[c];
   return ok;
 }
 
@@ -182,9 +197,10 @@ __device__ __forceinline__ void wide_visit(const DevScene& S, const Ray& r, cons
   for (int c = 0; c < 3; ++c) o[c] = __fmaf_rn(r.o[c], gs, -__uint_as_float(u0.x[c]));
   // time of the point closest to the cube's centre, in cube units
   const float tm = __fmaf_rn(o[0], w.w[0], __fmaf_rn(o[1], w.w[1], o[2] * w.w[2]));
-  const float slack = __fmaf_rn(fabsf(tm), 2.4e-7f, 1.f / 256);
-  const __half2 lo = __float2half2_rn(-tm - slack);
-  const __half2 hi = __float2half2_rn(__fmaf_rn(r.minT * w.dm, gs, slack - tm));
+  const __half2 lo =
+      __float2half2_rn(__fmaf_rn(kTEpsilon * w.dm, gs, -1.f / 256 - tm));
+  const __half2 hi = __float2half2_rn(__fmaf_rn(r.minT * w.dm, gs, 1.f / 256 - tm));
+  const __half2 far = __float2half2_rn(fabsf(tm) * kWide32);
   __half2 near01 = lo, near23 = lo, far01 = hi, far23 = hi;
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
@@ -200,8 +216,8 @@ __device__ __forceinline__ void wide_visit(const DevScene& S, const Ray& r, cons
     far23 = __hmin2(far23, __hfma2(h23, w.p2[c], t23));
   }
   int r0 = (int)u0.x[4], r1 = (int)u0.x[5], r2 = (int)u0.x[6], r3 = (int)u0.x[7];
-  keep_hit(near01, far01, r0, r1);
-  keep_hit(near23, far23, r2, r3);
+  keep_hit(near01, __hadd2(far01, far), r0, r1);
+  keep_hit(near23, __hadd2(far23, far), r2, r3);
   if (slots) {
     st.push_hit(r3);
     st.push_hit(r2);
@@ -284,7 +300,7 @@ __device__ __noinline__ Hit wide_trace_exact(const float4* nodes, const float4* 
 template <int KIND>
 __device__ __forceinline__ void wide_start(const DevScene& S, Ray& r, bool any, WideRay& w,
                                            Hit& h, int& ref, WideStack& st) {
-  const bool ok = wide_setup(S.origin_limit, r, any, w);
+  const bool ok = wide_setup(r, any, w) && wide_origin(S, r.o);
   int sp;
   start_ray(S, r, h, ref, sp);
   if (!ok && ref != kDone) {

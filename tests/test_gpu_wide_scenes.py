@@ -1,0 +1,104 @@
+"""Scenes and rays that the wide walk (rq_wide.cuh) must take at the binary walk's
+speed or better, and with its bits: far from the world's origin, with detail far
+finer than the whole, along axes and in the planes of the boxes."""
+import numpy as np
+import pytest
+
+from test_gpu_wide import _bits, _grid, _soup
+
+pytestmark = pytest.mark.gpu
+
+
+def _plan_pair(bvh, o, d, t, anyhit):
+    """A default plan and the binary walk's (register stack entries)."""
+    import torch
+    from rfmanta_b200.batch import BatchedQueries, QueryBatch
+    dev = [torch.from_numpy(np.ascontiguousarray(x, np.float32)).cuda() for x in (o, d, t)]
+    return [BatchedQueries([bvh], [QueryBatch(0, *dev, anyhit, want_uv=True)], cfg)
+            for cfg in (None, dict(reg_stack=1))]
+
+
+def _same_hits(bvh, o, d, t):
+    import torch
+    from rfmanta_b200.dynbvh import RayBatch
+    for anyhit in (False, True):
+        plans = _plan_pair(bvh, o, d, t, anyhit)
+        for p in plans:
+            p.launch()
+        torch.cuda.synchronize()
+        wide, binary = ([x[0].cpu().numpy() for x in (p.t, p.prim, p.u, p.v)] for p in plans)
+        r = RayBatch(o, d, t, flags=RayBatch.AnyHit if anyhit else 0)
+        bvh.intersect(r)
+        for a in (wide, [r.minT, r.hitPrim, r.u, r.v]):
+            assert np.array_equal(a[1], binary[1])
+            for i in (0, 2, 3):
+                assert np.array_equal(_bits(a[i]), _bits(binary[i]))
+        for p in plans:
+            p.close()
+    return int((binary[1] >= 0).sum())
+
+
+def _times(plans, reps=7):
+    import torch
+    out = []
+    for p in plans:
+        ms = []
+        for k in range(reps + 2):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            torch.cuda.synchronize()
+            a.record()
+            p.launch(torch.cuda.current_stream().cuda_stream)
+            b.record()
+            torch.cuda.synchronize()
+            ms.append(a.elapsed_time(b))
+        out.append(sorted(ms[2:])[reps // 2])
+    return out
+
+
+def _built(mesh, kind=0):
+    from rfmanta_b200.dynbvh import GpuDynBVH
+    b = GpuDynBVH(tri_kind=kind)
+    b.setGroup(mesh)
+    b.rebuild()
+    return b
+
+
+def _room_with_a_fine_sphere(radius):
+    from rfmanta_b200 import scenes
+    from rfmanta_b200.scenes import Mesh
+    v, f = scenes.icosphere(6)
+    room = np.array([[-3, -3, -3], [3, -3, -3], [3, 3, 3], [-3, 3, 3]], np.float64)
+    k = v.shape[0]
+    f = np.concatenate([f, [[k, k + 1, k + 2], [k, k + 2, k + 3]]]).astype(np.uint32)
+    return Mesh(np.concatenate([v * radius + 0.4, room]).astype(np.float32), f,
+                np.zeros(f.shape[0], np.uint32), np.full((1, 3), 0.5, np.float32))
+
+
+@pytest.mark.parametrize("case", ["off 100", "off 1000", "fine 3e-3", "fine 1e-3"])
+def test_far_and_fine_scenes_cost_what_others_do(case):
+    """The boxes' padding follows the ray, not the coordinates: within a factor of
+    two of the binary walk (the two differ by 0.7-0.9 near the origin; padding by
+    the coordinate cost 7 to 200 times here)."""
+    from rfmanta_b200 import scenes
+    rng = np.random.default_rng(5)
+    n = 1 << 17
+    if case.startswith("off"):
+        mesh = scenes.heightfield(256, 256, 7, extent=6.0)
+        mesh.vertices = (mesh.vertices.astype(np.float64) +
+                         [6.0 * float(case[4:]), 0.0, 2.0 * float(case[4:])]).astype(np.float32)
+        lo, hi = (x.astype(np.float64) for x in mesh.bounds())
+        o = lo + (hi - lo) * rng.random((n, 3))
+        d = rng.normal(size=(n, 3))
+    else:
+        mesh = _room_with_a_fine_sphere(float(case[5:]))
+        o = np.broadcast_to([-2.5, 2.0, 2.8], (n, 3))
+        d = mesh.vertices[rng.integers(0, mesh.vertices.shape[0] - 4, n)].astype(np.float64) - o
+    b = _built(mesh)
+    t = np.full(n, 1e19, np.float32)
+    assert _same_hits(b, o.T, d.T, t) > n // 4
+    plans = _plan_pair(b, o.T, d.T, t, False)
+    wide, binary = _times(plans)
+    assert wide < 2 * binary, (wide, binary)
+    for p in plans:
+        p.close()
+    b.close()
