@@ -37,8 +37,10 @@ static float bits_as_float(int32_t i) {
 
 // ------------------------------------------------------------ queries ----
 
+// (2^19 random closest hits over 65 instances at 72 / 80 / 96 registers: 312 / 290
+// / 307 us)
 template <int KIND, bool ANY, bool WIDE>
-__global__ void __launch_bounds__(128)
+__global__ void __maxnreg__(WIDE ? 80 : 128)
     trace2_kernel(DevScene T, const DevScene* blas, RayArgs a, int32_t* inst) {
   extern __shared__ int2 smem_stack[];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -54,7 +56,8 @@ __global__ void __launch_bounds__(128)
   r.minT = __ldg(a.tmax + i);
   Hit h;
   int ih, bh;
-  trace_two_level<KIND, ANY, false, WIDE>(T, blas, r, h, ih, bh, smem_stack + threadIdx.x, blockDim.x);
+  trace_two_level<KIND, ANY, false, WIDE, true>(T, blas, r, h, ih, bh, smem_stack + threadIdx.x,
+                                                blockDim.x);
   if (a.t) a.t[i] = h.t;
   if (a.prim) a.prim[i] = h.id;
   if (a.u) a.u[i] = h.u;
@@ -380,11 +383,10 @@ __device__ __forceinline__ void scene_trace(const DevScene& S, const DevScene* b
     st.init(reinterpret_cast<int*>(stk - threadIdx.x) + threadIdx.x, stride);
     WideRay w;
     int ref;
-    wide_start<KIND>(S, r, ANY, w, h, ref, st);
-    while (ref != kDone) {
-      while ((unsigned)ref < (unsigned)kDone) wide_visit(S, r, w, ANY, ref, st);
-      if (ref < 0) wide_leaf<KIND>(S, r, h, ANY, ref, st);
-    }
+    int sp;
+    start_ray(S, r, h, ref, sp);
+    const bool ok = ref != kDone && wide_setup(r, ANY, w);
+    wide_trace<KIND, ANY, false>(S, r, w, ok, h, ref, st);
     bh = -1;
   } else {
     int ref, sp;
@@ -407,8 +409,11 @@ __device__ __forceinline__ void add_counts(unsigned long long* dst, int a, int b
   }
 }
 
+// Registers of the wide forms: two-level frames 80 (1920x1080x4 at 72 / 80 / 96:
+// 2.21, 2.11, 2.15 ms), with reflections 96 (1280x720x4: 4.41, 4.36, 4.11 ms),
+// one-level frames 72 (72 / 80: 0.73, 0.75 ms).
 template <int KIND, bool TWO, bool STATS, bool WIDE>
-__global__ void __maxnreg__(72)
+__global__ void __maxnreg__(TWO && WIDE ? 80 : 72)
     frame_primary_kernel(DevScene S, const DevScene* blas, FrameParams P, SampleParams Q,
                          SampleBufs B, int n_items, unsigned long long* stats) {
   extern __shared__ int2 smem_stack[];
@@ -545,7 +550,7 @@ __device__ __forceinline__ float shade_hit(const DevScene& S, const DevScene* bl
 // in the reference's order (a reflection cut off by importance adds black
 // x reflectivity).
 template <int KIND, bool TWO, bool STATS, bool WIDE, bool REFL>
-__global__ void __maxnreg__(72)
+__global__ void __maxnreg__(!TWO || !WIDE ? 72 : REFL ? 96 : 80)
     frame_shade_kernel(DevScene S, const DevScene* blas, FrameParams P, SampleParams Q,
                        SampleBufs B, unsigned long long* stats) {
   extern __shared__ int2 smem_stack[];

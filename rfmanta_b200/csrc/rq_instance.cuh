@@ -16,8 +16,8 @@ namespace rq {
 // With STATS, cnt counts box tests (two per top-level record, one per root
 // box, the instance's included) and triangle tests.  WIDE: the inner scenes
 // are walked over their wide nodes, on a column of their own behind the
-// top-level entries (every inner tree has them).
-template <int KIND, bool ANY, bool STATS = false, bool WIDE = false>
+// top-level entries (every inner tree has them), FLAT as in wide_trace.
+template <int KIND, bool ANY, bool STATS = false, bool WIDE = false, bool FLAT = false>
 __device__ __forceinline__ void trace_two_level(const DevScene& T, const DevScene* blas,
                                                 Ray& r, Hit& h, int& inst_hit, int& blas_hit,
                                                 int2* stk, int stride, Counts* cnt = nullptr) {
@@ -97,20 +97,7 @@ __device__ __forceinline__ void trace_two_level(const DevScene& T, const DevScen
       if (STATS) cnt->boxes += 1;
       start_ray(S, lr, lh, lref, lsp);
       if (WIDE) {
-        if (lref != kDone && !(wide_ok && wide_origin(S, lr.o))) {
-          lh = wide_trace_exact<KIND, ANY>(S.nodes, S.tris, lref, lr);
-          lr.minT = lh.id >= 0 ? lh.t : lr.minT;
-          lref = kDone;
-        }
-        wst.reset();
-        DevScene L;
-        L.wide = S.wide;
-        L.tris = S.tris;
-        L.leaf_box = S.leaf_box;
-        while (lref != kDone) {
-          while ((unsigned)lref < (unsigned)kDone) wide_visit(L, lr, w, ANY, lref, wst);
-          if (lref < 0) wide_leaf<KIND>(L, lr, lh, ANY, lref, wst);
-        }
+        wide_trace<KIND, ANY, FLAT>(S, lr, w, wide_ok, lh, lref, wst);
       } else {
         while (lref != kDone)
           step<KIND, ANY, STATS>(S, lr, lh, lref, lsp, stk + sp * stride, stride, cnt);

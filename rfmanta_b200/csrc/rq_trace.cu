@@ -30,9 +30,14 @@ namespace rq {
 // idle lanes short (128 / 137 / 151 us for 777,777).
 constexpr int kClosestVote = 12, kAnyVote = 20;
 
+// Registers: 64 keep eight 128-thread blocks on an SM (uncapped, 70 or 64 with
+// spills: 777,777 random closest hits 171 us, capped 162; 3 M camera rays 204 and
+// 197).  Kensler-Shirley closest hits want 72 (camera rays 134 us, 143 at 64).
+constexpr int trace_registers(int kind) { return kind == kWald ? 64 : 72; }
+
 template <class Walk, bool ANY>
-__global__ void __launch_bounds__(256) trace_kernel(const __grid_constant__ DevScene S,
-                                                    RayArgs a) {
+__global__ void __maxnreg__(trace_registers(Walk::KIND))
+    trace_kernel(const __grid_constant__ DevScene S, RayArgs a) {
   extern __shared__ int2 smem_stack[];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   Walk walk;
@@ -54,7 +59,7 @@ __global__ void __launch_bounds__(256) trace_kernel(const __grid_constant__ DevS
 // idle (or none is busy), one lane claims that many ray indices with a single
 // atomicAdd and the idle lanes take them.
 template <class Walk, bool ANY>
-__global__ void __launch_bounds__(256)
+__global__ void __maxnreg__(trace_registers(Walk::KIND))
     trace_persistent_kernel(const __grid_constant__ DevScene S, RayArgs a, int* counter,
                             int refill) {
   extern __shared__ int2 smem_stack[];

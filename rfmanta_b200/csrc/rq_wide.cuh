@@ -48,10 +48,19 @@
 // visits but cost as many instructions a ray (more order to keep) and more L1
 // wavefronts; 8-bit boxes halve the bytes but need twice the padding.
 //
-// Rays outside these bounds (an infinite inverse direction, a slope above
-// kWideSlope, an origin more than kWideOrigin half sizes from the scene's centre)
-// take the exact
-// binary walk with a stack in local memory (wide_trace_exact).
+// Rays along an axis plane (a direction component of zero, or below 2^-kWideFlat of
+// the largest) are flat on that axis: their offset along it does not change, and
+// the slabs are tested with the slope kWideSlope (wide_visit<true>).  Where the
+// inverse is infinite and the origin lies on a plane of the hit leaf's box, the
+// exact tests of the boxes above it are not implied by the leaf's (0 * inf is NaN,
+// which bounds nothing): such a ray starts again on the exact walk, with what it
+// has found.
+//
+// Other rays outside the bounds (slopes between kWideSlope and flat, an origin
+// more than kWideOrigin half sizes from the scene's centre, no finite direction)
+// take the exact binary walk over the node records (exact_visit), in the same loop
+// and on the same stack column: refs alone, since a popped record's children are
+// tested against the minT of then.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -62,14 +71,20 @@ namespace rq {
 
 constexpr float kWidePad = 2.5e-3f;
 constexpr float kWide32 = 5e-7f;        // 8.4 * 2^-24
-constexpr float kWideSlope = 16384.f;   // largest |d|max / |d_k|
+constexpr float kWideSlope = 16384.f;   // |d|max / |d_k| is below
+constexpr int kWideFlat = 48;
 // Distance of an origin from the scene's centre in (largest) half sizes.  The
-// bound above needs kWideOrigin / kWideMinCube * kWide32 to stay a half number.
-constexpr float kWideOrigin = 64.f;
+// bound above needs kWideOrigin / kWideMinCube * kWide32 to stay a half number,
+// and a flat ray's real change of offset, 2^-kWideFlat of the distance in cubes,
+// to stay below kWidePad.  Camera rays from 400 / 1,000 / 1,900 sizes away on 295
+// k and 410 k triangles: 65 / 66 / 68 and 135 / 148 / 161 us (the exact walk: 72,
+// 74 and 193, 189 at the last two).
+constexpr float kWideOrigin = 4096.f;
 // Smallest cube over the scene's largest |coordinate|: 32 roundings of it, so
 // that the rounded centre is within 2/32 of the box's.
 constexpr float kWideMinCube = 1.f / (1 << 19);
-constexpr int kWideMaxDepth = 64;       // binary depth the local-memory stack takes
+// Deeper trees (chains, from files) keep the walk over the records.
+constexpr int kWideMaxDepth = 64;
 
 // What a wide visit needs of a ray beside the Ray itself.
 struct WideRay {
@@ -80,20 +95,26 @@ struct WideRay {
   __half2 n2[3];      // -|A|
   float dm;           // |d|max
   unsigned side;      // per folded record's byte: bit k: d_k > 0, bit 3 + k: not
-                      // (closest hit); all set: any hit
+                      // (closest hit); all set: any hit.  kRayFlat, kRayExact
 };
+constexpr unsigned kRayFlat = 1u << 24, kRayExact = 1u << 25;
 
 // Prepares a ray but for its origin; false when it must take the exact walk.
 __device__ __forceinline__ bool wide_setup(const Ray& r, bool any, WideRay& w) {
   const float ax = fabsf(r.d[0]), ay = fabsf(r.d[1]), az = fabsf(r.d[2]);
   w.dm = fmaxf(fmaxf(ax, ay), az);
-  bool ok = w.dm > 1e-15f && w.dm < 1e15f && !(r.minT != r.minT);
+  bool ok = w.dm > 1e-15f && w.dm < 1e15f && !(r.minT != r.minT), flat = false;
   const float rd = __fdividef(1.f, w.dm);
   float g[3], sum = 0.f;
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     w.A[c] = w.dm * r.inv[c];
-    ok = ok && fabsf(w.A[c]) <= kWideSlope;
+    if (fabsf(w.A[c]) > (float)(1LL << kWideFlat)) {
+      flat = true;
+      w.A[c] = kWideSlope;
+    } else {
+      ok = ok && fabsf(w.A[c]) < kWideSlope;
+    }
     g[c] = r.d[c] * rd;
     sum = __fmaf_rn(g[c], g[c], sum);
     w.a2[c] = __float2half2_rn(w.A[c]);
@@ -105,7 +126,7 @@ __device__ __forceinline__ bool wide_setup(const Ray& r, bool any, WideRay& w) {
   for (int c = 0; c < 3; ++c) w.w[c] = g[c] * k;
   const unsigned up =
       (r.d[0] > 0.f ? 1u : 0u) | (r.d[1] > 0.f ? 2u : 0u) | (r.d[2] > 0.f ? 4u : 0u);
-  w.side = 0x010101u * (any ? 0x3fu : up | (~up & 7u) << 3);
+  w.side = 0x010101u * (any ? 0x3fu : up | (~up & 7u) << 3) | (flat ? kRayFlat : 0u);
   return ok;
 }
 
@@ -186,7 +207,8 @@ struct WideStack {
 // One wide node: the children hit are pushed, last to visit first, and the
 // top of the stack (a child, or an older ref when none was hit) is popped.
 // slots: an any-hit ray, known where the code is compiled - its order is the
-// slots' own.
+// slots' own.  FLAT: the ray may be flat on some axis (told by its slope there).
+template <bool FLAT>
 __device__ __forceinline__ void wide_visit(const DevScene& S, const Ray& r, const WideRay& w,
                                            bool slots, int& ref, WideStack& st) {
   const char* p = reinterpret_cast<const char*>(S.wide) + 96 * (size_t)ref;
@@ -204,7 +226,8 @@ __device__ __forceinline__ void wide_visit(const DevScene& S, const Ray& r, cons
   __half2 near01 = lo, near23 = lo, far01 = hi, far23 = hi;
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    const __half2 b = __float2half2_rn(__fmaf_rn(-o[c], w.A[c], -tm));
+    const float at = FLAT && w.A[c] == kWideSlope ? 0.f : tm;
+    const __half2 b = __float2half2_rn(__fmaf_rn(-o[c], w.A[c], -at));
     const __half2 c01 = as_half2(c == 0 ? u1.x[0] : c == 1 ? u1.x[2] : u1.x[4]);
     const __half2 c23 = as_half2(c == 0 ? u1.x[1] : c == 1 ? u1.x[3] : u1.x[5]);
     const __half2 h01 = as_half2(c == 0 ? u1.x[6] : c == 1 ? u2.x[0] : u2.x[2]);
@@ -239,9 +262,9 @@ __device__ __forceinline__ void wide_visit(const DevScene& S, const Ray& r, cons
 
 // A leaf's triangles; the first accepted hit is preceded by the leaf's exact
 // box test with the minT the leaf was entered with.  Pops the next ref.
-template <int KIND>
-__device__ __forceinline__ void wide_leaf(const DevScene& S, Ray& r, Hit& h, bool any, int& ref,
-                                          WideStack& st) {
+template <int KIND, bool FLAT>
+__device__ __forceinline__ void wide_leaf(const DevScene& S, Ray& r, unsigned& side, Hit& h,
+                                          bool any, int& ref, WideStack& st) {
   const int first = ~ref;
   const float4* p = S.tris + 3 * (size_t)first;
   bool in_box = false;
@@ -260,6 +283,19 @@ __device__ __forceinline__ void wide_leaf(const DevScene& S, Ray& r, Hit& h, boo
                           __uint_as_float(b.x[2]), __uint_as_float(b.x[3]),
                           __uint_as_float(b.x[4]), __uint_as_float(b.x[5]), te);
         if (!in_box) break;
+        if (FLAT && (side & (kRayFlat | kRayExact)) == kRayFlat) {
+          bool on = false;
+#pragma unroll
+          for (int c = 0; c < 3; ++c)
+            on = on || (fabsf(r.inv[c]) == INFINITY && (r.o[c] == __uint_as_float(b.x[c]) ||
+                                                        r.o[c] == __uint_as_float(b.x[3 + c])));
+          if (on) {  // again from the root record (its root box was hit)
+            side |= kRayExact;
+            ref = 0;
+            st.reset();
+            return;
+          }
+        }
         r.minT = t_hit;
       }
       h = n;
@@ -275,55 +311,127 @@ __device__ __forceinline__ void wide_leaf(const DevScene& S, Ray& r, Hit& h, boo
   ref = st.pop();
 }
 
-// The exact binary walk to its end, for rays wide_setup refuses.  Arguments
-// and result by value: the callers' ray and hit stay in registers.
-template <int KIND, bool ANY>
-__device__ __noinline__ Hit wide_trace_exact(const float4* nodes, const float4* tris, int ref,
-                                             Ray r) {
-  DevScene S;
-  S.nodes = nodes;
-  S.tris = tris;
-  Hit h;
-  h.id = -1;
-  h.pos = -1;
-  h.t = r.minT;
-  h.u = h.v = 0.f;
-  int2 stk[kWideMaxDepth];
-  int sp = 0;
-  while (ref != kDone) step<KIND, ANY>(S, r, h, ref, sp, stk, 1);
-  return h;
+// One node record, with the exact tests, for rays outside the wide bounds.
+__device__ __forceinline__ void exact_visit(const DevScene& S, const Ray& r, bool fast, bool any,
+                                            int& ref, WideStack& st) {
+  const float4* p = S.nodes + 4 * (size_t)ref;
+  const float4 q0 = __ldg(p), q1 = __ldg(p + 1), q2 = __ldg(p + 2);
+  const int4 q3 = __ldg(reinterpret_cast<const int4*>(p + 3));
+  float tl, tr;
+  bool hl, hr;
+  box_pair(r, fast, q0, q1, q2, hl, hr, tl, tr);
+  if (hl && hr) {
+    const bool left_first = any ? ((q3.z >> 2) & 1) != 0 : pick3(r.d, q3.z & 3) > 0.f;
+    st.push_hit(left_first ? q3.y : q3.x);
+    ref = left_first ? q3.x : q3.y;
+  } else {
+    ref = hl ? q3.x : hr ? q3.y : st.pop();
+  }
 }
 
-// A ray's start: root box, and the whole exact walk where it must be taken.
-// ref = kDone when the ray is finished.  The column's first entry is the end
-// mark that the last pop returns.
-template <int KIND>
+// A lane's exact visits to its next leaf or its end, as the binary walk's step.
+__device__ __forceinline__ void exact_descend(const DevScene& S, const Ray& r, bool any, int& ref,
+                                              WideStack& st) {
+  const bool fast = inv_finite(r);
+  while ((unsigned)ref < (unsigned)kDone) exact_visit(S, r, fast, any, ref, st);
+}
+
+// A ray's start: root box and walk.  ref = kDone when the ray is finished.  The
+// column's first entry is the end mark that the last pop returns.
 __device__ __forceinline__ void wide_start(const DevScene& S, Ray& r, bool any, WideRay& w,
                                            Hit& h, int& ref, WideStack& st) {
-  const bool ok = wide_setup(r, any, w) && wide_origin(S, r.o);
   int sp;
   start_ray(S, r, h, ref, sp);
-  if (!ok && ref != kDone) {
-    h = any ? wide_trace_exact<KIND, true>(S.nodes, S.tris, ref, r)
-            : wide_trace_exact<KIND, false>(S.nodes, S.tris, ref, r);
-    ref = kDone;
-  }
+  if (ref == kDone) return;
+  if (!(wide_setup(r, any, w) && wide_origin(S, r.o))) w.side |= kRayExact;
   st.reset();
 }
 
+// The exact walk of a tree to its end, from `ref` on.  A call: inlined with its
+// loops in the two-level reflection kernel it took the frame from 4.2 to 5.0 ms.
+template <int KIND, bool ANY>
+__device__ __noinline__ Hit exact_trace(const float4* nodes, const float4* tris,
+                                        const float4* leaf_box, int ref, Ray r, Hit h,
+                                        WideStack st) {
+  DevScene S;
+  S.nodes = nodes;
+  for (;;) {
+    exact_descend(S, r, ANY, ref, st);
+    if (ref == kDone) return h;
+    const float4 a = __ldg(leaf_box + 2 * (size_t)(~ref));
+    const float4 b = __ldg(leaf_box + 2 * (size_t)(~ref) + 1);
+    float te;
+    if (box_test(r, a.x, a.y, a.z, a.w, b.x, b.y, te)) {
+      const float4* p = tris + 3 * (size_t)(~ref);
+      for (bool last = false; !last; p += 3) {
+        const bool hit = tri_test<KIND>(r, p, h, last);
+        if (hit) h.pos = (int)((p - tris) / 3);
+        if (ANY && hit) return h;
+      }
+    }
+    ref = st.pop();
+  }
+}
+
+// One lane's walk of a tree to its end, for kernels that trace a ray at a time,
+// its direction prepared (dir_ok: wide_setup's result).  FLAT: flat rays over the
+// wide nodes too; the frame kernels, whose pinhole and shadow rays are hardly ever
+// flat, send them to the exact walk and save the code.
+template <int KIND, bool ANY, bool FLAT>
+__device__ __forceinline__ void wide_trace(const DevScene& S, Ray& r, const WideRay& w,
+                                           bool dir_ok, Hit& h, int ref, WideStack& st) {
+  if (ref == kDone) return;
+  st.reset();
+  unsigned side = w.side;
+  if (dir_ok && (FLAT || !(side & kRayFlat)) && wide_origin(S, r.o)) {
+    DevScene L;
+    L.wide = S.wide;
+    L.tris = S.tris;
+    L.leaf_box = S.leaf_box;
+    do {
+      while ((unsigned)ref < (unsigned)kDone) wide_visit<FLAT>(L, r, w, ANY, ref, st);
+      if (ref < 0) wide_leaf<KIND, FLAT>(L, r, side, h, ANY, ref, st);
+    } while (ref != kDone && !(FLAT && (side & kRayExact)));
+    if (ref == kDone) return;
+  }
+  h = exact_trace<KIND, ANY>(S.nodes, S.tris, S.leaf_box, ref, r, h, st);
+  if (h.id >= 0) r.minT = h.t;
+}
+
 // Node visits of a whole warp until `vote` of its live lanes wait at a leaf
-// or at their end, then the waiting leaves.  Called by all 32 lanes.
-template <int KIND>
-__device__ __forceinline__ void wide_step(const DevScene& S, Ray& r, const WideRay& w, Hit& h,
-                                          bool any, bool live, int vote, bool slots,
-                                          int& ref, WideStack& st) {
+// or at their end.
+template <bool FLAT>
+__device__ __forceinline__ void wide_descend(const DevScene& S, const Ray& r, const WideRay& w,
+                                             bool live, int vote, bool slots, int& ref,
+                                             WideStack& st) {
   const int stop = max(0, __popc(__ballot_sync(0xffffffffu, live)) - vote);
   while (__popc(__ballot_sync(0xffffffffu, live && (unsigned)ref < (unsigned)kDone)) > stop) {
 #pragma unroll
     for (int k = 0; k < kWideVisits; ++k)
-      if (live && (unsigned)ref < (unsigned)kDone) wide_visit(S, r, w, slots, ref, st);
+      if (live && (unsigned)ref < (unsigned)kDone) wide_visit<FLAT>(S, r, w, slots, ref, st);
   }
-  if (live && ref < 0) wide_leaf<KIND>(S, r, h, any, ref, st);
+}
+
+// Flat rays are parallel as a rule and reach their leaves together: 3 M vertical
+// rays over 295 k triangles 271 -> 237 us against the caller's 12.
+constexpr int kFlatVote = 24;
+
+// wide_descend, then the leaves waiting.  Called by all 32 lanes.  A warp with
+// flat or exact rays takes loops of its own: the exact lanes go to their next
+// leaf first.
+template <int KIND>
+__device__ __forceinline__ void wide_step(const DevScene& S, Ray& r, WideRay& w, Hit& h,
+                                          bool any, bool live, int vote, bool slots,
+                                          int& ref, WideStack& st) {
+  if (__any_sync(0xffffffffu, live && w.side >= kRayFlat)) {
+    const bool exact = live && (w.side & kRayExact) != 0u;
+    if (exact) exact_descend(S, r, any, ref, st);
+    __syncwarp();
+    wide_descend<true>(S, r, w, live && !exact, max(vote, kFlatVote), slots, ref, st);
+  } else {
+    wide_descend<false>(S, r, w, live, vote, slots, ref, st);
+  }
+  if (live && ref < 0) wide_leaf<KIND, true>(S, r, w.side, h, any, ref, st);
 }
 
 // The two walks behind one interface, for kernels whose warps keep one ray per
@@ -365,7 +473,7 @@ struct WideWalk {
     st.init(static_cast<int*>(smem) + threadIdx.x, blockDim.x);
   }
   __device__ __forceinline__ void start(const DevScene& S, Ray& r, bool any, Hit& h, int& ref) {
-    wide_start<KIND>(S, r, any, w, h, ref, st);
+    wide_start(S, r, any, w, h, ref, st);
   }
   __device__ __forceinline__ void step(const DevScene& S, Ray& r, Hit& h, bool any, bool live,
                                        int vote, int& ref, bool slots = false) {
@@ -379,11 +487,10 @@ template <class Walk>
 __device__ __forceinline__ DevScene walk_scene(const DevScene& s) {
   DevScene S;
   S.tris = s.tris;
+  S.nodes = s.nodes;
   if (Walk::WIDE) {
     S.wide = s.wide;
     S.leaf_box = s.leaf_box;
-  } else {
-    S.nodes = s.nodes;
   }
   return S;
 }

@@ -102,3 +102,83 @@ def test_far_and_fine_scenes_cost_what_others_do(case):
     for p in plans:
         p.close()
     b.close()
+
+
+def _along_axes(mesh, seed, n=20000):
+    """Rays with one or two zero components (either sign, and components too small
+    to matter), origins exactly in the planes of the boxes and beside them, and
+    rays just outside the wide walk's slope and distance."""
+    rng = np.random.default_rng(seed)
+    v = mesh.vertices.astype(np.float64)
+    ext = max(float(np.ptp(v, axis=0).max()), 1e-3)
+    target = v[rng.integers(0, v.shape[0], n)]
+    mixed = rng.random((n, 1))
+    target = np.where(rng.random((n, 1)) < 0.5, target,
+                      mixed * target + (1 - mixed) * v[rng.integers(0, v.shape[0], n)])
+    d = rng.normal(size=(n, 3))
+    zero = rng.random((n, 3)) < 0.5
+    d = np.where(zero, rng.choice([0.0, -0.0, 1e-30, -1e-18], (n, 3)), d)
+    d[: n // 8] = rng.normal(size=(n // 8, 3)) * 10.0 ** -rng.uniform(0, 9, (n // 8, 3))
+    far = ext * np.where(rng.random((n, 1)) < 0.1, 1e4, rng.uniform(0, 3, (n, 1)))
+    o = target - d * far
+    o = np.where(np.abs(d) < 1e-12, target, o)  # in the plane of the target, exactly
+    t = rng.choice([1e19, np.inf, 3.0 * ext], n)
+    return [np.ascontiguousarray(x, np.float32) for x in (o.T, d.T, t)]
+
+
+def _boxes(n, seed):
+    """Faces of boxes at whole coordinates: planes shared by many nodes."""
+    from rfmanta_b200.scenes import Mesh
+    rng = np.random.default_rng(seed)
+    p = rng.integers(-6, 6, (n, 3))
+    q = p + rng.integers(0, 4, (n, 3))
+    tris = []
+    for a, b in zip(p, q):
+        k = int(rng.integers(0, 3))
+        u, w = (k + 1) % 3, (k + 2) % 3
+        c = np.array([a, a, a, a], np.float32)
+        c[1, u] = c[2, u] = b[u]
+        c[2, w] = c[3, w] = b[w]
+        tris += [c[[0, 1, 2]], c[[0, 2, 3]]]
+    v = np.concatenate(tris)
+    return Mesh(v, np.arange(v.shape[0], dtype=np.uint32).reshape(-1, 3),
+                np.zeros(2 * n, np.uint32), np.full((1, 3), 0.5, np.float32))
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("name", ["grid", "boxes", "soup", "far grid"])
+def test_rays_along_axes_and_in_the_boxes_planes(name, kind):
+    mesh = {"grid": lambda: _grid(24), "boxes": lambda: _boxes(400, 3),
+            "soup": lambda: _soup(500, 4),
+            "far grid": lambda: _grid(16, scale=0.25, offset=(4096.0, -512.0, 0.5))}[name]()
+    b = _built(mesh, kind)
+    for seed in (1, 2, 3):
+        assert _same_hits(b, *_along_axes(mesh, seed)) > 500
+    b.close()
+
+
+@pytest.mark.parametrize("case", ["vertical", "in planes", "along axes"])
+def test_rays_along_axes_cost_what_others_do(case):
+    """Below the binary walk, as other rays are (0.64-0.74 of it; the exact walk with
+    a stack in local memory, a whole ray at a time, cost 1.12-1.27)."""
+    from rfmanta_b200 import scenes
+    mesh = scenes.heightfield(256, 256, 7, extent=6.0)
+    rng = np.random.default_rng(6)
+    n = 1 << 20
+    lo, hi = (x.astype(np.float64) for x in mesh.bounds())
+    o = lo + (hi - lo) * rng.random((n, 3))
+    d = rng.normal(size=(n, 3))
+    if case == "vertical":
+        o[:, 1] = hi[1] + 1.0
+        d[:] = [0.0, -1.0, 0.0]
+    elif case == "in planes":
+        d[:, 1] = 0.0
+    else:
+        d = np.eye(3)[rng.integers(0, 3, n)]
+    b = _built(mesh)
+    plans = _plan_pair(b, o.T, d.T, np.full(n, 1e19, np.float32), False)
+    wide, binary = _times(plans)
+    assert wide < 0.95 * binary, (wide, binary)
+    for p in plans:
+        p.close()
+    b.close()
