@@ -90,9 +90,12 @@ constexpr int kBatchVote = 24;
 
 // SPLIT: the walk's stack is a SplitStack with a short shared column, and
 // registers are held to 48 per thread (five 256-thread blocks per SM), so
-// more warps are resident to hide the traversal's dependent loads.
+// more warps are resident to hide the traversal's dependent loads.  The wide
+// walk is held to 72 (seven 128-thread blocks): at its own 80, six blocks, 2^19
+// vertical rays took 103 us (88 at 72; binary walk 73), 3 M camera rays 267 (254;
+// 234), 3 M random ones 452 (431; 589).
 template <class Walk, bool SPLIT>
-__global__ void __launch_bounds__(256, SPLIT ? 5 : 1) batch_kernel(BatchArgs A) {
+__global__ void __maxnreg__(SPLIT ? 48 : Walk::WIDE ? 72 : 128) batch_kernel(BatchArgs A) {
   extern __shared__ int2 smem[];
   __shared__ DevScene sm_scenes[kMaxBatchScenes];
   for (int i = threadIdx.x; i < A.n_scenes; i += blockDim.x) sm_scenes[i] = A.scenes[i];

@@ -63,7 +63,9 @@ constexpr int kPathVote = 16;
 // Registers are capped so that seven (extend) and eight (shade) 128-thread
 // blocks fit an SM: uncapped the shade stage took 78-80 and six blocks (frame
 // 9.20 ms; shade at 72 / 64 registers 9.02 / 8.81, extend at 72 too 8.91 / 8.68,
-// extend at 56 spills: 9.04).
+// extend at 56 spills: 9.04).  The binary forms gain too, spills and all: a
+// 640x360x16 frame with 0 / 1 / 2 / 4 register stack entries 3.11 / 3.17 / 3.30 /
+// 3.41 ms uncapped, 2.97 / 3.03 / 3.05 / 3.07 capped.
 template <class Walk>
 __global__ void __maxnreg__(72)
     path_extend_persistent_kernel(DevScene S, PathParams P, PathBuffers B, int depth, int n0,
