@@ -974,7 +974,6 @@ int fail(int code, const std::string& msg) {
 }
 
 int cuda_fail(cudaError_t e, const char* what) {
-  cudaGetLastError();  // (a failed allocation is not the next launch's error)
   set_error(std::string("rotating update: ") + what + ": " + cudaGetErrorString(e));
   return e == cudaErrorMemoryAllocation ? RQ_ERR_OOM : RQ_ERR_CUDA;
 }

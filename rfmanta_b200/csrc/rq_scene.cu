@@ -28,7 +28,12 @@ namespace rq {
 
 static thread_local std::string g_error;
 
-void set_error(const std::string& msg) { g_error = msg; }
+void set_error(const std::string& msg) {
+  // what failed here is this call's error: the next call's launch checks must
+  // not find it
+  cudaGetLastError();
+  g_error = msg;
+}
 
 static thread_local int g_fail_allocation = 0;  // this one from now on fails, 0: none
 

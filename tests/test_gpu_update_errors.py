@@ -183,3 +183,28 @@ def test_a_plan_refuses_a_scene_that_lost_its_tree(nth):
     torch.cuda.synchronize()
     plan.close()
     b.close()
+
+
+@pytest.mark.gpu
+def test_a_refused_call_is_not_the_next_ones_error():
+    """Queries and frames of a tree whose stack does not fit are refused by the
+    runtime, on the host; the scene takes its next tree all the same."""
+    from rfmanta_b200 import _lib, scenes
+    from rfmanta_b200.dynbvh import GpuDynBVH
+    mesh, tree = _deep(LIMIT - 4)
+    b = GpuDynBVH()
+    b.setGroup(mesh)
+    b.rebuild()
+    blob = b.exportBlob()
+    want = _hits(b)
+    sc = scenes.tiny_frame_scene()
+    sc.mesh = mesh
+    for refused in (lambda: _hits(b), lambda: b.render_whitted(sc)):
+        b.importTree(tree)
+        with pytest.raises(_lib.RQError):
+            refused()
+        b.importBlob(blob)
+        b.update(rotate=True)
+        b.importBlob(blob)
+        assert np.array_equal(_hits(b).minT, want.minT)
+    b.close()
