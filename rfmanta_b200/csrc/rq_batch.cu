@@ -251,6 +251,7 @@ struct rq_batch_plan {
   std::vector<rq::Scene*> scenes;
   std::vector<uint64_t> generations;
   std::vector<rq::DevScene> host_scenes;
+  bool stale = false;  // host_scenes are ahead of the device's table or the graph
   int stack_depth = 1;
   bool wide = false;  // the captured kernel walks wide nodes
   int num_sms = 148;
@@ -291,6 +292,11 @@ int capture_plan(rq_batch_plan* p) {
   using namespace rq;
   const rq_batch_config& cfg = p->cfg;
   BatchArgs& A = p->args;
+  // (a plan whose capture fails has no graph until one succeeds)
+  if (p->exec) cudaGraphExecDestroy(p->exec);
+  if (p->graph) cudaGraphDestroy(p->graph);
+  p->exec = nullptr;
+  p->graph = nullptr;
   // split stack: the first smem_entries entries in shared memory, the rest
   // of the deepest tree's entries in the overflow area
   const bool split = cfg.smem_entries > 0;
@@ -333,10 +339,6 @@ int capture_plan(rq_batch_plan* p) {
     }
     A.ovf = p->d_ovf;
   }
-  if (p->exec) cudaGraphExecDestroy(p->exec);
-  if (p->graph) cudaGraphDestroy(p->graph);
-  p->exec = nullptr;
-  p->graph = nullptr;
   cudaError_t e = cudaStreamBeginCapture(p->cap_stream, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
     cudaMemsetAsync(p->d_counter, 0, sizeof(int), p->cap_stream);
@@ -500,7 +502,6 @@ int rq_batch_plan_create(rq_scene* const* scenes, int n_scenes, const rq_batch* 
 int rq_batch_plan_launch(rq_batch_plan* plan, void* stream) {
   if (!plan) return bfail(RQ_ERR_ARG, "NULL plan");
   if (cudaSetDevice(plan->device) != cudaSuccess) return bfail(RQ_ERR_CUDA, "cudaSetDevice");
-  bool changed = false;
   for (size_t i = 0; i < plan->scenes.size(); ++i) {
     rq::Scene* s = plan->scenes[i];
     if (s->generation == plan->generations[i]) continue;
@@ -509,18 +510,18 @@ int rq_batch_plan_launch(rq_batch_plan* plan, void* stream) {
     const int rc = s->node_layout(plan->cfg.node_layout, plan->host_scenes[i]);
     if (rc != RQ_OK) return rc;
     plan->generations[i] = s->generation;
-    changed = true;
+    plan->stale = true;
   }
-  if (changed) {
+  if (plan->stale) {  // and stays so until the table and the graph follow
     int depth = 1;
     for (const rq::DevScene& d : plan->host_scenes) depth = std::max(depth, d.depth);
     bool wide = plan->wide;
     for (const rq::DevScene& d : plan->host_scenes) wide = wide && d.wide;
-    if (depth > plan->stack_depth || wide != plan->wide) {
+    if (!plan->exec || depth > plan->stack_depth || wide != plan->wide) {
       // a deeper tree, or one without wide nodes: a larger stack or the
       // binary walk, captured again (after the launches already queued, which
       // still use the old graph)
-      plan->stack_depth = std::max(depth, plan->stack_depth);
+      plan->stack_depth = depth;
       const int rc = capture_plan(plan);
       if (rc != RQ_OK) return rc;
     }
@@ -531,6 +532,7 @@ int rq_batch_plan_launch(rq_batch_plan* plan, void* stream) {
                         sizeof(rq::DevScene) * plan->host_scenes.size(), cudaMemcpyHostToDevice,
                         static_cast<cudaStream_t>(stream));
     if (c != cudaSuccess) return bfail(RQ_ERR_CUDA, "scene table");
+    plan->stale = false;
   }
   const cudaError_t e = cudaGraphLaunch(plan->exec, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return bfail(RQ_ERR_CUDA, std::string("graph launch: ") + cudaGetErrorString(e));

@@ -208,3 +208,39 @@ def test_a_refused_call_is_not_the_next_ones_error():
         b.importBlob(blob)
         assert np.array_equal(_hits(b).minT, want.minT)
     b.close()
+
+
+@pytest.mark.gpu
+def test_a_plan_waits_for_a_tree_it_can_take():
+    """A tree too deep for the plan's stack is an error at every launch (the old
+    graph would read the freed tree), and the plan runs again with the next one."""
+    import torch
+    from rfmanta_b200 import _lib, scenes
+    from rfmanta_b200.batch import BatchedQueries, QueryBatch
+    from rfmanta_b200.dynbvh import GpuDynBVH
+    mesh, tree = _deep(LIMIT - 4)
+    b = GpuDynBVH()
+    b.setGroup(mesh)
+    b.rebuild()
+    blob = b.exportBlob()
+    o, d, _, _ = scenes.random_rays(4096, np.full(3, -1.0), np.full(3, 1.0), seed=7,
+                                    anyhit_fraction=0.0)
+    q = QueryBatch(0, *(torch.from_numpy(x).cuda() for x in (o, d)),
+                   torch.full((o.shape[1],), 1e19, device="cuda"))
+    plan = BatchedQueries([b], [q])
+    plan.launch()
+    torch.cuda.synchronize()
+    want = [plan.t[0].cpu().numpy(), plan.prim[0].cpu().numpy()]
+    b.importTree(tree)
+    for _ in range(2):
+        with pytest.raises(_lib.RQError) as e:
+            plan.launch()
+        assert e.value.code == _lib.RQ_ERR_CAPACITY
+    b.importBlob(blob)
+    plan.t[0].zero_()
+    plan.launch()
+    torch.cuda.synchronize()
+    for got, w in zip((plan.t[0].cpu().numpy(), plan.prim[0].cpu().numpy()), want):
+        assert np.array_equal(got, w)
+    plan.close()
+    b.close()
