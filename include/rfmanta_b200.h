@@ -214,6 +214,10 @@ RQ_API int rq_scene_sah_cost(const rq_scene* scene, double* cost);
 RQ_API int rq_scene_info(const rq_scene* scene, int* n_records, int* n_leaves,
                   int* depth, size_t* device_bytes);
 
+/* Whether queries and frames of the scene walk the four-wide nodes of its tree
+ * (two-level: of the inner trees) rather than its node records. */
+RQ_API int rq_scene_walks_wide(const rq_scene* scene, int* wide);
+
 /*
  * Exports the tree in the saveToFile byte format (DynBVH::saveToFile).
  * With blob == NULL only *bytes is set.
@@ -456,6 +460,8 @@ RQ_API int rq_batch_plan_create(rq_scene* const* scenes, int n_scenes,
                                 const rq_batch_config* cfg, rq_batch_plan** out);
 /* Replays the plan's graph on `stream` (a cudaStream_t; NULL = legacy). */
 RQ_API int rq_batch_plan_launch(rq_batch_plan* plan, void* stream);
+/* Whether the plan's last launch (or its creation) walked four-wide nodes. */
+RQ_API int rq_batch_plan_walks_wide(const rq_batch_plan* plan, int* wide);
 RQ_API int rq_batch_plan_info(const rq_batch_plan* plan, rq_batch_config* cfg,
                               int* grid, long long* total_rays);
 RQ_API int rq_batch_plan_destroy(rq_batch_plan* plan);

@@ -214,6 +214,8 @@ def _load():
         "rq_scene_update_vertices_device": ([vp, vp, i, i, vp], i),
         "rq_scene_update_state": ([vp, vp, i, vp], i),
         "rq_fail_allocation": ([i], i),
+        "rq_scene_walks_wide": ([vp, C.POINTER(i)], i),
+        "rq_batch_plan_walks_wide": ([vp, C.POINTER(i)], i),
         "rq_mesh_read_ply": ([C.c_char_p, vp, C.c_uint32, C.POINTER(vp)], i),
         "rq_mesh_info": ([vp, C.POINTER(i), C.POINTER(i)], i),
         "rq_mesh_copy": ([vp, vp, vp, vp], i),

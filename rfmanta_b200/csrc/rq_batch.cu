@@ -285,6 +285,15 @@ rq_batch_config default_batch_config() {
   return c;
 }
 
+// Whether the plan's scenes and configuration take the wide walk: register
+// entries, a split stack, another record order (node_layout clears the
+// descriptors' wide nodes) and counted tests are the binary walk's.
+bool plan_wide(const rq_batch_plan* p) {
+  bool wide = p->cfg.smem_entries == 0 && p->cfg.reg_stack == 0 && !p->args.stats;
+  for (const rq::DevScene& d : p->host_scenes) wide = wide && d.wide;
+  return wide;
+}
+
 // Sizes the traversal stack for the plan's deepest tree and captures
 // counter reset + persistent launch in a graph (again after a scene's tree
 // grew deeper).
@@ -303,10 +312,7 @@ int capture_plan(rq_batch_plan* p) {
   const int reg = split ? kSplitStack : cfg.reg_stack;
   A.stack_depth = split ? std::min(cfg.smem_entries, p->stack_depth) : p->stack_depth;
   // the shared-memory column holds what the register entries do not
-  // (register entries, a split stack, another record order and counted tests
-  // are the binary walk's; node_layout clears the descriptors' wide nodes)
-  p->wide = !split && cfg.reg_stack == 0 && A.stats == nullptr;
-  for (const DevScene& d : p->host_scenes) p->wide = p->wide && d.wide;
+  p->wide = plan_wide(p);
   p->smem = stack_bytes(A.stack_depth, cfg.block_threads, p->wide, split ? 0 : cfg.reg_stack);
   const void* f = batch_fn(p->tri_kind, reg, p->wide, A.stats != nullptr);
   if (p->smem > 0 &&
@@ -515,12 +521,10 @@ int rq_batch_plan_launch(rq_batch_plan* plan, void* stream) {
   if (plan->stale) {  // and stays so until the table and the graph follow
     int depth = 1;
     for (const rq::DevScene& d : plan->host_scenes) depth = std::max(depth, d.depth);
-    bool wide = plan->wide;
-    for (const rq::DevScene& d : plan->host_scenes) wide = wide && d.wide;
-    if (!plan->exec || depth > plan->stack_depth || wide != plan->wide) {
-      // a deeper tree, or one without wide nodes: a larger stack or the
-      // binary walk, captured again (after the launches already queued, which
-      // still use the old graph)
+    if (!plan->exec || depth > plan->stack_depth || plan_wide(plan) != plan->wide) {
+      // a deeper tree, or trees that lost or got back their wide nodes: a
+      // larger stack or the other walk, captured again (after the launches
+      // already queued, which still use the old graph)
       plan->stack_depth = depth;
       const int rc = capture_plan(plan);
       if (rc != RQ_OK) return rc;
@@ -536,6 +540,12 @@ int rq_batch_plan_launch(rq_batch_plan* plan, void* stream) {
   }
   const cudaError_t e = cudaGraphLaunch(plan->exec, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return bfail(RQ_ERR_CUDA, std::string("graph launch: ") + cudaGetErrorString(e));
+  return RQ_OK;
+}
+
+int rq_batch_plan_walks_wide(const rq_batch_plan* plan, int* wide) {
+  if (!plan || !wide) return bfail(RQ_ERR_ARG, "NULL argument");
+  *wide = plan->exec && plan->wide ? 1 : 0;
   return RQ_OK;
 }
 

@@ -682,6 +682,12 @@ int rq_scene_info(const rq_scene* s, int* n_records, int* n_leaves, int* depth,
   return RQ_OK;
 }
 
+int rq_scene_walks_wide(const rq_scene* s, int* wide) {
+  if (!s || !wide) return fail(RQ_ERR_ARG, "NULL argument");
+  *wide = s->has_tree && (s->instanced ? s->inner_wide() : s->dev().wide != nullptr) ? 1 : 0;
+  return RQ_OK;
+}
+
 int rq_trace_device(rq_scene* s, int n, const float* d_org, const float* d_dir,
                     const float* d_tmax, int flags, float* d_t, int32_t* d_prim,
                     float* d_u, float* d_v, void* stream) {

@@ -143,7 +143,7 @@ struct Scene {
   uint64_t generation = 0;
   std::vector<uint64_t> blas_generation;  // two-level: inner generations at creation
   int check_inner_current() const;
-  bool inner_wide() const;  // two-level: the inner trees can be walked wide
+  bool inner_wide() const;  // two-level: the inner trees are walked wide
 
   rq_launch_config cfg[4];  // RQ_CLOSEST, RQ_ANYHIT, RQ_PATH_EXTEND, RQ_PATH_SHADE
   int* d_counter = nullptr;  // persistent-launch counters for rq_trace_device

@@ -161,8 +161,8 @@ def test_wide_walk_is_the_binary_walk(name, kind):
 
 
 def test_trees_the_wide_walk_refuses():
-    """Boxes that are not nested, and a tree deeper than the exact walk's
-    stack: both are traced as before, over the node records."""
+    """Boxes that are not nested, and a tree deeper than the wide walk takes:
+    both are traced as before, over the node records."""
     from rfmanta_b200.dynbvh import GpuDynBVH
     from rfmanta_b200.treeio import TreeFields, parse_dynbvh_blob
     mesh = _soup(300, 9)

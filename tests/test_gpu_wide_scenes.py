@@ -182,3 +182,107 @@ def test_rays_along_axes_cost_what_others_do(case):
     for p in plans:
         p.close()
     b.close()
+
+
+def _walks_wide(scene=None, plan=None):
+    import ctypes as C
+    from rfmanta_b200 import _lib
+    w = C.c_int(-1)
+    if plan is not None:
+        _lib.check(_lib.lib.rq_batch_plan_walks_wide(plan._plan, C.byref(w)))
+    else:
+        _lib.check(_lib.lib.rq_scene_walks_wide(scene.handle, C.byref(w)))
+    return bool(w.value)
+
+
+def _far(mesh):
+    mesh.vertices = (mesh.vertices + np.float32(1e4)).astype(np.float32)
+    return mesh
+
+
+@pytest.mark.parametrize("name", ["one", "two", "three", "five", "soup", "flat", "small far away",
+                                  "doubled", "sphere", "heightfield", "far", "fine"])
+def test_which_trees_are_walked_wide(name):
+    """Every tree of more than one leaf, after a build and after each update, and
+    the default plan over it; the comparisons of test_gpu_wide.py compare two
+    walks only if this holds."""
+    from test_gpu_wide import _meshes
+    mesh = dict(_meshes()).get(name) or {"far": lambda: _far(_grid(9)),
+                                         "fine": lambda: _room_with_a_fine_sphere(1e-3)}[name]()
+    b = _built(mesh)
+    o = np.zeros((3, 8), np.float32)
+    plans = _plan_pair(b, o, o + 1, np.ones(8, np.float32), False)
+    many = b.info().n_records > 0
+    assert many == (name != "one")
+    assert _walks_wide(b) == many
+    assert [_walks_wide(plan=p) for p in plans] == [many, False]
+    for rotate in (True, False, True) if many else ():
+        mesh.vertices = (mesh.vertices * np.float32(1.01)).astype(np.float32)
+        b.update(rotate=rotate)
+        assert _walks_wide(b) == (b.info().n_records > 0)
+        for p in plans:
+            p.launch()
+        assert [_walks_wide(plan=p) for p in plans] == [b.info().n_records > 0, False]
+    for p in plans:
+        p.close()
+    b.close()
+
+
+def test_a_plan_follows_its_scene_to_the_records_and_back():
+    """Boxes that are not nested send scene and plan to the binary walk; the next
+    tree brings both back."""
+    import torch
+    from rfmanta_b200.treeio import parse_dynbvh_blob
+    mesh = _soup(300, 9)
+    b = _built(mesh)
+    blob = b.exportBlob()
+    t = parse_dynbvh_blob(blob, mesh.n_tris)
+    inner = np.nonzero((t.children == 0) & (np.arange(t.children.shape[0]) > 0))[0]
+    for i in inner[:20]:
+        c = (t.bounds[i, :3] + t.bounds[i, 3:]) / 2
+        t.bounds[i] = np.concatenate([c, c]) + 0.4 * (t.bounds[i] - np.concatenate([c, c]))
+    o, d, tmax = _along_axes(mesh, 3, 4000)
+    p = _plan_pair(b, o, d, tmax, False)
+    p[1].close()
+    p = p[0]
+    p.launch()
+    torch.cuda.synchronize()
+    want = p.prim[0].cpu().numpy()
+    assert _walks_wide(b) and _walks_wide(plan=p)
+    b.importTree(t)
+    p.launch()
+    assert not _walks_wide(b) and not _walks_wide(plan=p)
+    b.importBlob(blob)
+    p.launch()
+    torch.cuda.synchronize()
+    assert _walks_wide(b) and _walks_wide(plan=p)
+    assert np.array_equal(p.prim[0].cpu().numpy(), want)
+    p.close()
+    b.close()
+
+
+@pytest.mark.parametrize("case,wide", [("alike", True), ("far", True), ("tiny", False),
+                                       ("one triangle", False)])
+def test_which_two_level_scenes_are_walked_wide(case, wide):
+    """Inner trees wherever they lie, unless one has no wide nodes or is so small
+    that rays reach it from beyond its origins' limit."""
+    from rfmanta_b200 import scenes
+    from rfmanta_b200.dynbvh import InstancedBVH
+    mesh = scenes.displaced_icosphere(3, seed=6)
+    if case == "far":
+        mesh = _far(mesh)
+    if case == "tiny":
+        mesh.vertices = (mesh.vertices * np.float32(1e-3)).astype(np.float32)
+    if case == "one triangle":
+        mesh = _soup(1, 1)
+    inner = [_built(mesh), _built(scenes.heightfield(12, 10, 5, extent=3.0))]
+    move = np.array([[0, 0, 0], [0, 0, 0], [3, 0.5, 1], [-2, 1, 2]], np.float32)
+    if case == "far":
+        move[[0, 2, 3]] -= np.float32(1e4)
+    top = InstancedBVH(inner, np.array([0, 1, 0, 0], np.int32), move,
+                       np.array([0, 1, 0, 0], np.int32))
+    top.rebuild()
+    assert _walks_wide(top) == wide
+    top.close()
+    for b in inner:
+        b.close()
