@@ -210,7 +210,9 @@ RQ_API int rq_mesh_materials(const rq_mesh* mesh, int32_t* kind, float* diffuse,
 /* SAH cost of the scene's tree, DynBVH::computeCost<>(0) with C_isec=C_trav=1. */
 RQ_API int rq_scene_sah_cost(const rq_scene* scene, double* cost);
 
-/* Counts: internal records, leaves, maximum traversal depth. */
+/* Counts: internal records, leaves, maximum traversal depth; device_bytes: what
+ * mesh and tree hold on the device (164 bytes a record, 84 a triangle of the tree;
+ * scratch of frames and updates not counted). */
 RQ_API int rq_scene_info(const rq_scene* scene, int* n_records, int* n_leaves,
                   int* depth, size_t* device_bytes);
 

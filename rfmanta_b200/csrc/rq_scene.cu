@@ -676,9 +676,18 @@ int rq_scene_info(const rq_scene* s, int* n_records, int* n_leaves, int* depth,
   if (n_records) *n_records = s->n_records;
   if (n_leaves) *n_leaves = s->n_leaves;
   if (depth) *depth = s->depth;
-  if (device_bytes)
-    *device_bytes = (size_t)s->n_records * 64 + (size_t)s->n_leaf_tris * 48 +
-                    s->verts.size() * 4 + s->idx.size() * 4 + s->face_mat.size() * 4;
+  if (device_bytes) {
+    size_t tree = 0;
+    if (s->has_tree && s->instanced) {
+      tree = (size_t)s->n_records * 64 + s->inst_blas.size() * 2 * sizeof(float4);
+    } else if (s->has_tree) {
+      // d_nodes, d_level_recs, d_tris (set_tree); the update's arrays are extra
+      const int cap = std::max(s->rec_capacity, 1);
+      tree = rq::Scene::record_bytes(cap) + (size_t)cap * 4 +
+             (size_t)s->n_leaf_tris * (48 + 32 + 4);
+    }
+    *device_bytes = tree + s->verts.size() * 4 + s->idx.size() * 4 + s->face_mat.size() * 4;
+  }
   return RQ_OK;
 }
 

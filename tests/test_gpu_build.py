@@ -95,3 +95,27 @@ def test_degenerate_inputs():
                      np.array([[0.0], [0.0], [-1.0]], np.float32))
         bvh.intersect(r)
         assert r.hitPrim[0] >= 0 and abs(float(r.minT[0]) - 1.0) < 1e-6
+
+
+def test_device_bytes_are_what_the_scene_holds():
+    """rq_scene_info's figure against the device memory that making the scene took
+    (the allocator's grain, 2 MB a block, aside)."""
+    import torch
+    from rfmanta_b200 import scenes
+    from rfmanta_b200.dynbvh import GpuDynBVH
+    mesh = scenes.heightfield(700, 700, 3, extent=6.0)
+    torch.cuda.synchronize()
+    warm = GpuDynBVH()
+    warm.setGroup(scenes.heightfield(8, 8, 3, extent=6.0))
+    warm.rebuild()
+    b = GpuDynBVH()
+    b.setGroup(mesh)
+    before = torch.cuda.mem_get_info()[0]
+    b.rebuild()
+    torch.cuda.synchronize()
+    took = before - torch.cuda.mem_get_info()[0]
+    said = b.info().device_bytes
+    assert said > 100 << 20
+    assert abs(took - said) < (32 << 20), (took, said)
+    b.close()
+    warm.close()
