@@ -1408,9 +1408,8 @@ def run_ours(args):
         if others:
             line["other_workloads"] = others
         if not args.no_cpu_baseline and world == 1:  # the host baseline: rank 0 at N=1
-            v, threads, text, _ = wl.cpu_reference(args.cpu_seconds, os.cpu_count() or 1)
-            line["cpu_baseline"] = {"value": round(v, 3), "unit": "Mrays/s", "cores": threads,
-                                    "kind": "reference", "sample": text}
+            threads = os.cpu_count() or 1
+            line["cpu_baseline"] = host_baseline(wl, args.cpu_seconds, threads)
             if hasattr(wl, "image_check"):
                 line["image_error"] = wl.image_check()
             if wl.name in ("path_frame", "small_frame"):
@@ -1421,6 +1420,20 @@ def run_ours(args):
         print(json.dumps(line), flush=True)
     if world > 1:
         dist.destroy_process_group()
+
+
+NO_REFERENCE = "oracle/_ref/libmanta_ref.so was not built (needs the reference sources)"
+
+
+def host_baseline(wl, seconds, threads):
+    """The line's cpu_baseline: the reference on the host cores, or why not (the
+    device's figures stand without it)."""
+    from oracle.pyoracle import Reference
+    if not (Reference.available() or Reference.available(sse=True)):
+        return {"kind": "reference", "unavailable": NO_REFERENCE}
+    v, threads, text, _ = wl.cpu_reference(seconds, threads)
+    return {"value": round(v, 3), "unit": "Mrays/s", "cores": threads, "kind": "reference",
+            "sample": text}
 
 
 def run_custom(args, wl, dev, world, rank):
@@ -1447,9 +1460,7 @@ def run_custom(args, wl, dev, world, rank):
             "roofline": None,
         }
         if not args.no_cpu_baseline and world == 1:  # the host baseline: rank 0 at N=1
-            v, threads, text, _ = wl.cpu_reference(args.cpu_seconds, os.cpu_count() or 1)
-            line["cpu_baseline"] = {"value": round(v, 3), "unit": "Mrays/s", "cores": threads,
-                                    "kind": "reference", "sample": text}
+            line["cpu_baseline"] = host_baseline(wl, args.cpu_seconds, os.cpu_count() or 1)
         print(json.dumps(line), flush=True)
     if world > 1:
         dist.destroy_process_group()
@@ -1478,8 +1489,7 @@ def run_reference(args):
         return
     from oracle.pyoracle import Reference
     if not Reference.available():
-        print(json.dumps({"impl": "reference", "unavailable":
-                          "oracle/_ref/libmanta_ref.so was not built (needs the reference sources)"}))
+        print(json.dumps({"impl": "reference", "unavailable": NO_REFERENCE}))
         return
     wl = make_workload(args)
     threads = os.cpu_count() or 1
