@@ -55,7 +55,9 @@ struct PathBuffers {
   int* tile_counts;  // scratch of the ordered compaction
   unsigned long long* ray_counts;  // [0] extension rays, [1] shadow rays
   unsigned long long* stats;       // optional box/tri test counters (4)
-  // optional per-bounce dump for parity checks: [depth][path]
+  // optional per-bounce dump for parity checks: [depth][dbg_paths], the caller's
+  // count (the buffers above may hold more)
+  size_t dbg_paths;
   int32_t* dbg_prim;
   float* dbg_org;  // [3][depth][path]
   float* dbg_dir;

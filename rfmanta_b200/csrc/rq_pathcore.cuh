@@ -107,17 +107,17 @@ __device__ __forceinline__ void load_extension_ray(const PathBuffers& B, int p, 
 __device__ __forceinline__ void store_extension(const PathParams& P, const PathBuffers& B,
                                                 int depth, int p, const Ray& r,
                                                 const Hit& h) {
-  const size_t C = B.capacity;
   B.t[p] = h.t;
   B.pos[p] = h.pos;
   B.prim[p] = h.id;
   if (B.dbg_prim) {
-    const size_t k = (size_t)depth * C + p;
+    const size_t k = (size_t)depth * B.dbg_paths + p;
+    const size_t rows = (size_t)P.max_depth * B.dbg_paths;
     B.dbg_prim[k] = h.id;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      B.dbg_org[(size_t)c * P.max_depth * C + k] = r.o[c];
-      B.dbg_dir[(size_t)c * P.max_depth * C + k] = r.d[c];
+      B.dbg_org[c * rows + k] = r.o[c];
+      B.dbg_dir[c * rows + k] = r.d[c];
     }
   }
 }

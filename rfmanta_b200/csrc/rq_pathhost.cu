@@ -246,6 +246,7 @@ static int path_run(Scene* s, const PathParams& P, long long total, int chunk, f
   B.dbg_prim = s->path_dbg_prim;
   B.dbg_org = s->path_dbg_org;
   B.dbg_dir = s->path_dbg_dir;
+  B.dbg_paths = (size_t)s->path_dbg_capacity;
   if (B.dbg_prim && (long long)s->path_dbg_capacity < total)
     return pfail(RQ_ERR_ARG, "debug buffers smaller than the frame's path count");
   if (B.dbg_prim && chunk != total) return pfail(RQ_ERR_ARG, "debug dump needs a single chunk");

@@ -100,3 +100,27 @@ def test_debug_dumps_are_one_pass_of_at_most_4_mi_paths(tiny):
             assert e.value.code == _lib.RQ_ERR_ARG
             b.render_path(sc, chunk_paths=n)  # one pass by the caller's choice
         b.set_path_debug(0, 0, 0, 0)
+
+
+def test_a_dump_after_a_larger_frame(tiny):
+    """The dump's rows are as long as the caller says, whatever the buffers hold."""
+    import torch
+    from rfmanta_b200 import scenes
+    sc, b = tiny
+    n, D = sc.xres * sc.yres * sc.spp, sc.max_depth
+
+    def dump(cap):
+        pad = 1 << 16  # behind each array: must stay as it is
+        prim = torch.full((D * cap + pad,), -2, dtype=torch.int32, device="cuda")
+        od = [torch.full((3 * D * cap + pad,), -2.0, device="cuda") for _ in range(2)]
+        b.set_path_debug(prim.data_ptr(), od[0].data_ptr(), od[1].data_ptr(), cap)
+        b.render_path(sc)
+        b.set_path_debug(0, 0, 0, 0)
+        assert all(bool((x[-pad:] == -2).all()) for x in (prim, *od))
+        return [x[:-pad].cpu().numpy().reshape(-1, cap)[:, :n] for x in (prim, *od)]
+
+    want = dump(n)
+    b.render_path(scenes.tiny_path_scene(150, 100, 16))
+    for cap in (n, n + 5):
+        for got, w in zip(dump(cap), want):
+            assert np.array_equal(got, w)
