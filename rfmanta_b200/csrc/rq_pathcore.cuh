@@ -122,21 +122,6 @@ __device__ __forceinline__ void store_extension(const PathParams& P, const PathB
   }
 }
 
-// Closest hit of one live path's current ray.
-template <int KIND, bool STATS>
-__device__ __forceinline__ void extend_path(const DevScene& S, const PathParams& P,
-                                            const PathBuffers& B, int depth, int p,
-                                            int2* stk, int stride, Counts& cnt) {
-  Ray r;
-  load_extension_ray(B, p, r);
-  Hit h;
-  int ref, sp;
-  start_ray(S, r, h, ref, sp);
-  if (STATS) cnt.boxes = 1;
-  while (ref != kDone) step<KIND, false, STATS>(S, r, h, ref, sp, stk, stride, &cnt);
-  store_extension(P, B, depth, p, r, h);
-}
-
 // First half of one live path's bounce: background on a miss, else BSDF
 // sample, the light sample and Russian roulette, with the path's next state
 // (o, d, importance, RNG) written when it survives.  When the light sample
@@ -311,28 +296,6 @@ __device__ __forceinline__ void shade_finish(const PathBuffers& B, int p,
   const size_t C = B.capacity;
 #pragma unroll
   for (int c = 0; c < 3; ++c) B.rad[c * C + p] = fadd(B.rad[c * C + p], contrib[c]);
-}
-
-// One live path at one bounce in one thread: shade_begin, the any-hit
-// shadow ray, shade_finish.  Returns true when the path continues.
-template <int KIND, bool STATS>
-__device__ __forceinline__ bool shade_path(const DevScene& S, const PathParams& P,
-                                           const PathBuffers& B, int depth, int p,
-                                           long long g, int2* stk, int stride, Counts& cnt,
-                                           int& nshadow) {
-  Ray sr;
-  float contrib[3];
-  bool alive;
-  if (shade_begin<KIND>(S, P, B, depth, p, g, sr, contrib, alive)) {
-    ++nshadow;
-    Hit sh;
-    int ref, sp;
-    start_ray(S, sr, sh, ref, sp);
-    if (STATS) cnt.boxes += 1;
-    while (ref != kDone) step<KIND, true, STATS>(S, sr, sh, ref, sp, stk, stride, &cnt);
-    if (sh.id < 0) shade_finish(B, p, contrib);
-  }
-  return alive;
 }
 
 }  // namespace rq
