@@ -24,19 +24,24 @@
 namespace rq {
 
 // Wide walk: lanes of a warp that wait at a leaf, or have ended, before the
-// others stop descending.  Random rays, bound by L1 wavefronts, want the
-// leaves batched (closest hit 209 / 189 / 184 us at 8 / 16 / 24 for 2^20 rays,
-// any hit 507 / 427 / 404 us for 3 M), camera rays, bound by issue slots, the
-// idle lanes short (128 / 137 / 151 us for 777,777).
+// others stop descending.  Random rays, bound by L1 wavefronts, want the leaves
+// batched (any hit 507 / 427 / 404 us at 8 / 16 / 24 for 3 M; closest hits at 12 /
+// 16 / 20: 359 / 333 / 326 us for 3 M over 8 k triangles), sparse camera rays,
+// bound by issue slots, the idle lanes short (closest 150 / 157 / 158 us for
+// 777,777 over 410 k).  Any-hit rays end at their first hit and lose nothing at
+// 20; closest hits stay at 12 for the camera's sake.  A vote that follows what
+// the warp sees is not built.
 constexpr int kClosestVote = 12, kAnyVote = 20;
 
-// Registers: 64 keep eight 128-thread blocks on an SM (uncapped, 70 or 64 with
-// spills: 777,777 random closest hits 171 us, capped 162; 3 M camera rays 204 and
-// 197).  Kensler-Shirley closest hits want 72 (camera rays 134 us, 143 at 64).
-constexpr int trace_registers(int kind) { return kind == kWald ? 64 : 72; }
+// Registers of both forms: left alone the compiler takes 64 for closest Wald hits
+// and spills (777,777 random rays over 295 k triangles 171 us, 160 at 72).  At 64
+// without spills batches of millions gain 2-4% (3 M camera rays over 8 k triangles
+// 145 -> 140 us) and small ones, bound by latency, lose 3-8% (100 k over 295 k
+// 33.9 -> 35.9 us); Kensler-Shirley rays lose 6% (777,777 camera rays 134 -> 143).
+constexpr int kTraceRegisters = 72;
 
 template <class Walk, bool ANY>
-__global__ void __maxnreg__(trace_registers(Walk::KIND))
+__global__ void __maxnreg__(kTraceRegisters)
     trace_kernel(const __grid_constant__ DevScene S, RayArgs a) {
   extern __shared__ int2 smem_stack[];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -59,7 +64,7 @@ __global__ void __maxnreg__(trace_registers(Walk::KIND))
 // idle (or none is busy), one lane claims that many ray indices with a single
 // atomicAdd and the idle lanes take them.
 template <class Walk, bool ANY>
-__global__ void __maxnreg__(trace_registers(Walk::KIND))
+__global__ void __maxnreg__(kTraceRegisters)
     trace_persistent_kernel(const __grid_constant__ DevScene S, RayArgs a, int* counter,
                             int refill) {
   extern __shared__ int2 smem_stack[];
