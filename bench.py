@@ -236,10 +236,10 @@ class PathFrame:
     # launches (bounces 0-3) of one full-size frame of this workload
     # (1280x720x16, 26.5M extension rays), summed over the launches and
     # divided by their rays.
-    DRAM_BYTES_PER_RAY = 72.9
+    DRAM_BYTES_PER_RAY = 72.5
     DRAM_BASIS = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the 4 "
-                  "path_extend_persistent_kernel launches of one full-size frame (1.934 GB "
-                  "over 26,534,621 extension rays = 72.9 B per ray) x extension rays per "
+                  "path_extend_persistent_kernel launches of one full-size frame (1.923 GB "
+                  "over 26,534,621 extension rays = 72.5 B per ray) x extension rays per "
                   "launch (all bounces / depth)")
 
     def traffic(self, rays):
@@ -257,9 +257,9 @@ class PathFrame:
     # instruction.
     LIMITER = {"limiter": "issue slots at half-full warps and dependent-load latency, "
                           "not HBM bandwidth",
-               "lanes_per_warp_instruction": 16.8, "warps_active_pct": 38.4,
-               "warps_active_theoretical_pct": 50.0, "issue_active_pct": 58.0,
-               "l1tex_throughput_pct": 54.6, "l2_throughput_pct": 8.5,
+               "lanes_per_warp_instruction": 16.9, "warps_active_pct": 38.3,
+               "warps_active_theoretical_pct": 50.0, "issue_active_pct": 57.4,
+               "l1tex_throughput_pct": 53.4, "l2_throughput_pct": 7.5,
                "long_scoreboard_stalls_per_issue": 5.49,
                "profile": "profiles/wide_walk_kernels.md"}
 
@@ -630,12 +630,12 @@ class CoherentFrame:
 
     # DRAM bytes per primary ray of frame_primary_kernel, from one ncu
     # capture of this workload at 960x540 x 1 spp (518,400 rays, same scene).
-    DRAM_BYTES_PER_RAY = 182.0
+    DRAM_BYTES_PER_RAY = 176.9
 
     def traffic(self, rays):
         prim, _ = rays
         return self.DRAM_BYTES_PER_RAY * prim, ("ncu DRAM bytes per primary ray at 960x540x1 "
-                                                "(182.0 B) x primary rays of the launch")
+                                                "(176.9 B) x primary rays of the launch")
 
     def group_stages(self, stage_ms):
         return self.stage_names, [stage_ms[0], stage_ms[1], stage_ms[2]]
@@ -779,7 +779,7 @@ class BatchedQueriesWL:
     # kind of configuration (wide walk), scaled to a full launch by its rays
     # (the batches and scenes are the same, so the re-read pattern per ray
     # carries over).
-    DRAM_BYTES_PER_RAY = 247.7
+    DRAM_BYTES_PER_RAY = 234.3
 
     # What bounds batch_kernel, from the ncu counters of that launch.
     LIMITER = {"limiter": "L1 wavefronts and load latency of uniformly random rays, "

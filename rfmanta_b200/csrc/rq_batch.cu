@@ -85,7 +85,10 @@ struct BatchWide : WideWalk<KIND_> {
 };
 
 // Wide walk: lanes waiting at a leaf or at their end before the others stop
-// descending; 24 batches of random rays at 8 / 12 / 16 / 24: 615 / 570 / 543 / 530 us.
+// descending; 24 batches of random rays at 8 / 12 / 16 / 24: 615 / 570 / 543 / 530
+// us, 3 M camera rays at 8 / 12 / 16 / 20 / 24: 279 / 269 / 257 / 255 / 254 (kinds
+// and scenes mix in a warp here, so the leaves' batching counts more than in
+// rq_trace.cu's kernels).
 constexpr int kBatchVote = 24;
 
 // SPLIT: the walk's stack is a SplitStack with a short shared column, and

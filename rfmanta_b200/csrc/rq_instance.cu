@@ -327,7 +327,8 @@ struct SampleBufs {
 //
 // Sample of work item k: a warp's 32 items are the samples of a tile of pixels
 // (8x4, 4x2 or 2x1 at 1, 4 or 16 samples) where those tiles cover the image, else
-// 32 consecutive samples.
+// 32 consecutive samples (1921x1081x4 without tiles 2.145 ms, 1920x1080x4 with
+// them 2.12).
 __device__ __forceinline__ int item_sample(const FrameParams& P, const SampleParams& Q, int k) {
   const int tw = Q.spp == 1 ? 8 : Q.spp == 4 ? 4 : 2, th = Q.spp == 1 ? 4 : Q.spp == 4 ? 2 : 1;
   if (Q.spp * tw * th != 32 || P.xres % tw || P.yres % th) return k;

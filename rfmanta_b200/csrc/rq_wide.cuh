@@ -42,11 +42,14 @@
 // visits, reads a node in three loads for a record's four, and votes: a warp
 // stops descending once enough lanes wait at leaves, so leaves are tested by
 // more lanes together.  Measured against the binary walk: 777,777 camera rays
-// 241 -> 136 us, 2^20 random closest hits 243 -> 199 us, 3 M random occlusion
-// rays 583 -> 399 us, the 512x512 Whitted frame 214 -> 128 us, the 1280x720x16
-// path frame 11.38 -> 8.68 ms (7.31 in one pass, rq_pathhost.cu).  Eight-wide nodes would save a third more
-// visits but cost as many instructions a ray (more order to keep) and more L1
-// wavefronts; 8-bit boxes halve the bytes but need twice the padding.
+// 234 -> 134 us, 2^20 random closest hits 239 -> 194 us, 3 M random occlusion
+// rays 581 -> 385 us, the 512x512 Whitted frame 211 -> 133 us, the 1280x720x16
+// path frame 11.35 -> 7.24 ms (in one pass, rq_pathhost.cu).  Dense coherent
+// closest hits, two to four visits a ray, lose by their longer setup: 3 M camera
+// rays over 8 k / 295 k triangles 122 -> 145, 174 -> 203 us.  Eight-wide nodes
+// would save a third more visits but cost as many instructions a ray (more order
+// to keep) and more L1 wavefronts; 8-bit boxes halve the bytes but need twice the
+// padding.
 //
 // Rays along an axis plane (a direction component of zero, or below 2^-kWideFlat of
 // the largest) are flat on that axis: their offset along it does not change, and
