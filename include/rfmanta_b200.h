@@ -70,8 +70,8 @@ RQ_API const char* rq_version(void);
 
 /*
  * For tests of what callers see when memory is short: the nth device
- * allocation that this host thread's tree imports, updates and path frames
- * make from now on fails on the host (RQ_ERR_OOM); 0 takes the failure back.  Other threads
+ * allocation that this host thread's tree imports, updates and frames make
+ * from now on fails on the host (RQ_ERR_OOM); 0 takes the failure back.  Other threads
  * and calls are not affected.
  */
 RQ_API int rq_fail_allocation(int nth);

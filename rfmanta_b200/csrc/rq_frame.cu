@@ -132,17 +132,16 @@ static int prepare(Scene* s, const rq_whitted_params* p, FrameParams& P) {
     return set_fail(RQ_ERR_ARG, "bad environment (kind, or a zero background up)");
   if (!s->frame) s->frame = new FrameScratch();
   FrameScratch* f = s->frame;
-  if (!f->counters) {
-    if (cudaMalloc(&f->counters, kNumCounters * sizeof(int)) != cudaSuccess ||
-        cudaMalloc(&f->shadow, sizeof(unsigned long long)) != cudaSuccess)
-      return set_fail(RQ_ERR_OOM, "frame counters allocation failed");
-  }
+  if ((!f->counters && !device_array(&f->counters, kNumCounters)) ||
+      (!f->shadow && !device_array(&f->shadow, 1)))
+    return set_fail(RQ_ERR_OOM, "frame counters allocation failed");
   const float* mrgb = p->material_rgb;
   if (f->n_materials != p->n_materials ||
       std::memcmp(f->host_materials.data(), mrgb, sizeof(float) * 3 * p->n_materials) != 0) {
     cudaFree(f->materials);
     f->materials = nullptr;
-    if (cudaMalloc(&f->materials, sizeof(float) * 3 * p->n_materials) != cudaSuccess)
+    f->n_materials = 0;
+    if (!device_array(&f->materials, 3 * (size_t)p->n_materials))
       return set_fail(RQ_ERR_OOM, "materials allocation failed");
     if (cudaMemcpy(f->materials, mrgb, sizeof(float) * 3 * p->n_materials,
                    cudaMemcpyHostToDevice) != cudaSuccess)
@@ -216,9 +215,9 @@ int rq_render_whitted(rq_scene* scene, const rq_whitted_params* params, float* r
     cudaFree(f->d_prim);
     f->d_rgb = f->d_t = nullptr;
     f->d_prim = nullptr;
-    if (cudaMalloc(&f->d_rgb, npix * 12) != cudaSuccess ||
-        cudaMalloc(&f->d_t, npix * 4) != cudaSuccess ||
-        cudaMalloc(&f->d_prim, npix * 4) != cudaSuccess)
+    f->out_npix = 0;
+    if (!rq::device_array(&f->d_rgb, 3 * npix) || !rq::device_array(&f->d_t, npix) ||
+        !rq::device_array(&f->d_prim, npix))
       return rq::set_fail(RQ_ERR_OOM, "frame output allocation failed");
     f->out_npix = npix;
   }

@@ -789,25 +789,26 @@ int frame_prepare(rq::Scene* s, const rq_frame_params* fp, rq::FrameParams& P,
   if (x->items < items) {
     x->free_items();
     SampleBufs& B = x->B;
-    if (cudaMalloc(&B.t, 4 * items) != cudaSuccess || cudaMalloc(&B.prim, 4 * items) != cudaSuccess ||
-        cudaMalloc(&B.pos, 4 * items) != cudaSuccess || cudaMalloc(&B.blas, 4 * items) != cudaSuccess ||
-        cudaMalloc(&B.col, 12 * items) != cudaSuccess || cudaMalloc(&B.queue, 4 * items) != cudaSuccess ||
-        cudaMalloc(&B.hit, items) != cudaSuccess ||
-        cudaMalloc(&B.tiles, 4 * (size_t)flag_compaction_tiles((int)items)) != cudaSuccess) {
+    if (!device_array(&B.t, items) || !device_array(&B.prim, items) ||
+        !device_array(&B.pos, items) || !device_array(&B.blas, items) ||
+        !device_array(&B.col, 3 * items) || !device_array(&B.queue, items) ||
+        !device_array(&B.hit, items) ||
+        !device_array(&B.tiles, (size_t)flag_compaction_tiles((int)items))) {
       x->free_items();
       return ifail(RQ_ERR_OOM, "frame sample buffers");
     }
     x->items = items;
   }
-  if (!x->B.counters && (cudaMalloc(&x->B.counters, 16) != cudaSuccess ||
-                         cudaMalloc(&x->B.shadow, 8) != cudaSuccess))
+  if ((!x->B.counters && !device_array(&x->B.counters, 4)) ||
+      (!x->B.shadow && !device_array(&x->B.shadow, 1)))
     return ifail(RQ_ERR_OOM, "frame counters");
   const float* mrgb = p->material_rgb;
   if ((int)x->host_materials.size() != 3 * p->n_materials ||
       std::memcmp(x->host_materials.data(), mrgb, sizeof(float) * 3 * p->n_materials) != 0) {
     cudaFree(x->materials);
     x->materials = nullptr;
-    if (cudaMalloc(&x->materials, 12 * (size_t)p->n_materials) != cudaSuccess ||
+    x->host_materials.clear();
+    if (!device_array(&x->materials, 3 * (size_t)p->n_materials) ||
         cudaMemcpy(x->materials, mrgb, 12 * (size_t)p->n_materials, cudaMemcpyHostToDevice) != cudaSuccess)
       return ifail(RQ_ERR_OOM, "materials");
     x->host_materials.assign(mrgb, mrgb + 3 * p->n_materials);
@@ -827,7 +828,8 @@ int frame_prepare(rq::Scene* s, const rq_frame_params* fp, rq::FrameParams& P,
         std::memcmp(x->host_phong.data(), ph.data(), ph.size() * sizeof(float4)) != 0) {
       cudaFree(x->phong);
       x->phong = nullptr;
-      if (cudaMalloc(&x->phong, ph.size() * sizeof(float4)) != cudaSuccess ||
+      x->host_phong.clear();
+      if (!device_array(&x->phong, ph.size()) ||
           cudaMemcpy(x->phong, ph.data(), ph.size() * sizeof(float4), cudaMemcpyHostToDevice) !=
               cudaSuccess)
         return ifail(RQ_ERR_OOM, "Phong table");
@@ -846,7 +848,8 @@ int frame_prepare(rq::Scene* s, const rq_frame_params* fp, rq::FrameParams& P,
     if (x->host_refl != rf) {
       cudaFree(x->refl);
       x->refl = nullptr;
-      if (cudaMalloc(&x->refl, rf.size() * sizeof(float)) != cudaSuccess ||
+      x->host_refl.clear();
+      if (!device_array(&x->refl, rf.size()) ||
           cudaMemcpy(x->refl, rf.data(), rf.size() * sizeof(float), cudaMemcpyHostToDevice) !=
               cudaSuccess)
         return ifail(RQ_ERR_OOM, "reflectivity table");
@@ -910,7 +913,8 @@ int rq_render_frame(rq_scene* scene, const rq_frame_params* params, float* rgb,
   if (x->rgb_pix < npix) {
     cudaFree(x->d_rgb);
     x->d_rgb = nullptr;
-    if (cudaMalloc(&x->d_rgb, 12 * npix) != cudaSuccess) return rq::ifail(RQ_ERR_OOM, "image");
+    x->rgb_pix = 0;
+    if (!rq::device_array(&x->d_rgb, 3 * npix)) return rq::ifail(RQ_ERR_OOM, "image");
     x->rgb_pix = npix;
   }
   rc = frame_run(s, P, Q, x->d_rgb, nullptr, x->stream);

@@ -60,6 +60,10 @@ cudaError_t launch_flag_compaction(const uint8_t* flags, int n, int* tile_counts
 
 // cudaMalloc, with rq_fail_allocation's failures.
 cudaError_t device_alloc(void** p, size_t bytes);
+template <class T>
+bool device_array(T** p, size_t n) {
+  return device_alloc(reinterpret_cast<void**>(p), (n ? n : 1) * sizeof(T)) == cudaSuccess;
+}
 
 void set_error(const std::string& msg);
 

@@ -129,11 +129,6 @@ static int pfail(int code, const std::string& m) {
   return code;
 }
 
-template <class T>
-static bool palloc(T** p, size_t n) {
-  return cudaMalloc(reinterpret_cast<void**>(p), std::max<size_t>(n, 1) * sizeof(T)) == cudaSuccess;
-}
-
 static bool recording(cudaStream_t st) {
   cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
   if (!st || cudaStreamIsCapturing(st, &c) != cudaSuccess) {
@@ -220,12 +215,12 @@ static int path_prepare(Scene* s, const rq_path_params* p, PathParams& P, long l
     ps->was_short = true;
     parts *= 2;
   }
-  if (!ps->counts && !palloc(&ps->counts, 2)) return pfail(RQ_ERR_OOM, "counter allocation");
+  if (!ps->counts && !device_array(&ps->counts, 2)) return pfail(RQ_ERR_OOM, "counter allocation");
   const float* mrgb = p->material_rgb;
   if ((int)ps->host_materials.size() != 3 * p->n_materials ||
       std::memcmp(ps->host_materials.data(), mrgb, sizeof(float) * 3 * p->n_materials) != 0) {
     ps->free_materials();
-    if (!palloc(&ps->materials, 3 * (size_t)p->n_materials) ||
+    if (!device_array(&ps->materials, 3 * (size_t)p->n_materials) ||
         cudaMemcpy(ps->materials, mrgb, sizeof(float) * 3 * p->n_materials,
                    cudaMemcpyHostToDevice) != cudaSuccess)
       return pfail(RQ_ERR_OOM, "materials upload failed");
@@ -311,7 +306,8 @@ int rq_render_path(rq_scene* scene, const rq_path_params* params, float* rgb,
   if (ps->rgb_pix < npix) {
     cudaFree(ps->d_rgb);
     ps->d_rgb = nullptr;
-    if (!rq::palloc(&ps->d_rgb, 3 * npix)) return rq::pfail(RQ_ERR_OOM, "image allocation");
+    ps->rgb_pix = 0;
+    if (!rq::device_array(&ps->d_rgb, 3 * npix)) return rq::pfail(RQ_ERR_OOM, "image allocation");
     ps->rgb_pix = npix;
   }
   rc = rq::path_run(s, P, total, chunk, ps->d_rgb, nullptr, ps->stream);

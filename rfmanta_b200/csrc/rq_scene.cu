@@ -733,6 +733,8 @@ int rq_trace(rq_scene* s, int n, const float* org, const float* dir,
       const size_t cap = 11 * (size_t)rq::kZeroCopyRays * sizeof(float);
       if (cudaHostAlloc(&st->h_map, cap, cudaHostAllocMapped) != cudaSuccess ||
           cudaHostGetDevicePointer(&st->d_map, st->h_map, 0) != cudaSuccess) {
+        if (st->h_map) cudaFreeHost(st->h_map);
+        st->h_map = nullptr;
         s->release(st);
         return fail(RQ_ERR_OOM, "mapped staging allocation failed");
       }
