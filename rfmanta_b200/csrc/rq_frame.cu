@@ -83,6 +83,8 @@ struct FrameScratch {
   int32_t* counters = nullptr;
   unsigned long long* shadow = nullptr;
   float* materials = nullptr;
+  bool materials_recorded = false;  // a frame in a CUDA graph holds them
+  Kept kept;
   int n_materials = 0;
   std::vector<float> host_materials;
   // host-output staging
@@ -109,7 +111,7 @@ static int set_fail(int code, const std::string& m) {
   return code;
 }
 
-static int prepare(Scene* s, const rq_whitted_params* p, FrameParams& P) {
+static int prepare(Scene* s, const rq_whitted_params* p, FrameParams& P, cudaStream_t st) {
   if (!p) return set_fail(RQ_ERR_ARG, "NULL params");
   if (p->xres <= 0 || p->yres <= 0 || (long long)p->xres * p->yres > (1LL << 30))
     return set_fail(RQ_ERR_ARG, "bad resolution");
@@ -138,7 +140,7 @@ static int prepare(Scene* s, const rq_whitted_params* p, FrameParams& P) {
   const float* mrgb = p->material_rgb;
   if (f->n_materials != p->n_materials ||
       std::memcmp(f->host_materials.data(), mrgb, sizeof(float) * 3 * p->n_materials) != 0) {
-    cudaFree(f->materials);
+    f->kept.give_up(f->materials, f->materials_recorded);
     f->materials = nullptr;
     f->n_materials = 0;
     if (!device_array(&f->materials, 3 * (size_t)p->n_materials))
@@ -150,6 +152,7 @@ static int prepare(Scene* s, const rq_whitted_params* p, FrameParams& P) {
     f->n_materials = p->n_materials;
   }
   P.materials = f->materials;
+  f->materials_recorded = f->materials_recorded || recording(st);
   return RQ_OK;
 }
 
@@ -189,7 +192,7 @@ int rq_render_whitted_device(rq_scene* scene, const rq_whitted_params* params, f
   if (cudaSetDevice(s->device) != cudaSuccess) return rq::set_fail(RQ_ERR_CUDA, "cudaSetDevice");
   std::lock_guard<std::mutex> g(s->frame_mu);
   rq::FrameParams P;
-  int rc = rq::prepare(s, params, P);
+  int rc = rq::prepare(s, params, P, static_cast<cudaStream_t>(stream));
   if (rc != RQ_OK) return rc;
   return rq::launch(s, P, d_rgb, d_t, d_prim,
                     reinterpret_cast<unsigned long long*>(d_shadow_rays),
@@ -203,7 +206,7 @@ int rq_render_whitted(rq_scene* scene, const rq_whitted_params* params, float* r
   if (cudaSetDevice(s->device) != cudaSuccess) return rq::set_fail(RQ_ERR_CUDA, "cudaSetDevice");
   std::lock_guard<std::mutex> g(s->frame_mu);
   rq::FrameParams P;
-  int rc = rq::prepare(s, params, P);
+  int rc = rq::prepare(s, params, P, nullptr);
   if (rc != RQ_OK) return rc;
   rq::FrameScratch* f = s->frame;
   const size_t npix = (size_t)params->xres * params->yres;

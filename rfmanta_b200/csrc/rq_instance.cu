@@ -720,11 +720,17 @@ struct SampleScratch {
   float* d_rgb = nullptr;
   size_t rgb_pix = 0;
   cudaStream_t stream = nullptr;
+  // what a frame in a CUDA graph holds
+  bool items_recorded = false, materials_recorded = false, phong_recorded = false,
+       refl_recorded = false;
+  Kept kept;
   void free_items() {
-    cudaFree(B.t); cudaFree(B.prim); cudaFree(B.pos); cudaFree(B.blas); cudaFree(B.col);
-    cudaFree(B.queue);
-    cudaFree(B.hit);
-    cudaFree(B.tiles);
+    for (void* p : {(void*)B.t, (void*)B.prim, (void*)B.pos, (void*)B.blas, (void*)B.col,
+                    (void*)B.queue, (void*)B.hit, (void*)B.tiles}) {
+      bool recorded = items_recorded;
+      kept.give_up(p, recorded);
+    }
+    items_recorded = false;
     B.t = B.col = nullptr;
     B.prim = B.pos = B.blas = B.queue = B.tiles = nullptr;
     B.hit = nullptr;
@@ -749,7 +755,7 @@ void destroy_sample_scratch(SampleScratch* p) { delete p; }
 namespace {
 
 int frame_prepare(rq::Scene* s, const rq_frame_params* fp, rq::FrameParams& P,
-                  rq::SampleParams& Q) {
+                  rq::SampleParams& Q, cudaStream_t st) {
   using namespace rq;
   if (!fp) return ifail(RQ_ERR_ARG, "NULL params");
   const rq_whitted_params* p = &fp->whitted;
@@ -805,7 +811,7 @@ int frame_prepare(rq::Scene* s, const rq_frame_params* fp, rq::FrameParams& P,
   const float* mrgb = p->material_rgb;
   if ((int)x->host_materials.size() != 3 * p->n_materials ||
       std::memcmp(x->host_materials.data(), mrgb, sizeof(float) * 3 * p->n_materials) != 0) {
-    cudaFree(x->materials);
+    x->kept.give_up(x->materials, x->materials_recorded);
     x->materials = nullptr;
     x->host_materials.clear();
     if (!device_array(&x->materials, 3 * (size_t)p->n_materials) ||
@@ -826,7 +832,7 @@ int frame_prepare(rq::Scene* s, const rq_frame_params* fp, rq::FrameParams& P,
     }
     if (x->host_phong.size() != ph.size() ||
         std::memcmp(x->host_phong.data(), ph.data(), ph.size() * sizeof(float4)) != 0) {
-      cudaFree(x->phong);
+      x->kept.give_up(x->phong, x->phong_recorded);
       x->phong = nullptr;
       x->host_phong.clear();
       if (!device_array(&x->phong, ph.size()) ||
@@ -846,7 +852,7 @@ int frame_prepare(rq::Scene* s, const rq_frame_params* fp, rq::FrameParams& P,
       return ifail(RQ_ERR_ARG, "max_depth must be in [0, 32]");
     std::vector<float> rf(fp->material_reflectivity, fp->material_reflectivity + p->n_materials);
     if (x->host_refl != rf) {
-      cudaFree(x->refl);
+      x->kept.give_up(x->refl, x->refl_recorded);
       x->refl = nullptr;
       x->host_refl.clear();
       if (!device_array(&x->refl, rf.size()) ||
@@ -858,6 +864,11 @@ int frame_prepare(rq::Scene* s, const rq_frame_params* fp, rq::FrameParams& P,
     P.refl = x->refl;
     P.max_depth = fp->max_depth;
     P.cutoff = fp->importance_cutoff;
+  }
+  if (recording(st)) {
+    x->items_recorded = x->materials_recorded = true;
+    x->phong_recorded = x->phong_recorded || P.phong;
+    x->refl_recorded = x->refl_recorded || P.refl;
   }
   return RQ_OK;
 }
@@ -891,7 +902,7 @@ int rq_render_frame_device(rq_scene* scene, const rq_frame_params* params, float
   std::lock_guard<std::mutex> g(s->frame_mu);
   rq::FrameParams P;
   rq::SampleParams Q;
-  int rc = frame_prepare(s, params, P, Q);
+  int rc = frame_prepare(s, params, P, Q, static_cast<cudaStream_t>(stream));
   if (rc != RQ_OK) return rc;
   return frame_run(s, P, Q, d_rgb, d_shadow_rays, static_cast<cudaStream_t>(stream));
 }
@@ -904,7 +915,7 @@ int rq_render_frame(rq_scene* scene, const rq_frame_params* params, float* rgb,
   std::lock_guard<std::mutex> g(s->frame_mu);
   rq::FrameParams P;
   rq::SampleParams Q;
-  int rc = frame_prepare(s, params, P, Q);
+  int rc = frame_prepare(s, params, P, Q, nullptr);
   if (rc != RQ_OK) return rc;
   rq::SampleScratch* x = s->samples;
   const size_t npix = (size_t)P.xres * P.yres;

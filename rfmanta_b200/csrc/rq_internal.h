@@ -5,6 +5,7 @@
 
 #include <cstdint>
 #include <string>
+#include <vector>
 
 #include "rq_device.cuh"
 
@@ -64,6 +65,26 @@ template <class T>
 bool device_array(T** p, size_t n) {
   return device_alloc(reinterpret_cast<void**>(p), (n ? n : 1) * sizeof(T)) == cudaSuccess;
 }
+
+// Whether the stream is being recorded into a CUDA graph.
+bool recording(cudaStream_t st);
+
+// Device memory that frames recorded into a caller's CUDA graph may hold: given
+// up by an owner that replaces it, such memory is kept until the owner goes (at
+// most one block per recording), other memory is freed.
+struct Kept {
+  std::vector<void*> blocks;
+  void give_up(void* p, bool& recorded) {
+    if (recorded && p)
+      blocks.push_back(p);
+    else
+      cudaFree(p);
+    recorded = false;
+  }
+  ~Kept() {
+    for (void* p : blocks) cudaFree(p);
+  }
+};
 
 void set_error(const std::string& msg);
 

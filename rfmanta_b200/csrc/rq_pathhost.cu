@@ -37,34 +37,22 @@ struct PathScratch {
   // All of B's buffers in one allocation: 13 cost 4.5 ms and as much to free,
   // one 0.4-0.8 ms (80 MB to 2.4 GB).
   void* memory = nullptr;
-  // A frame recorded into a CUDA graph holds B's pointers, so such buffers are
-  // kept until the scene goes when a larger frame replaces them (at most one
-  // set per recorded size: capacities only grow).
-  bool recorded = false;
-  std::vector<void*> retired;
+  // A frame recorded into a CUDA graph holds B's pointers and the material
+  // table's.
+  bool recorded = false, materials_recorded = false;
+  Kept kept;
   // An allocation failed: frames fit their passes to the buffers there are
   // instead of failing it again each time.
   bool was_short = false;
-  // The recorded kernels read the material table too; one they hold is kept
-  // in the same way when a frame brings other materials.
-  bool materials_recorded = false;
   void free_materials() {
-    if (materials_recorded)
-      retired.push_back(materials);
-    else
-      cudaFree(materials);
+    kept.give_up(materials, materials_recorded);
     materials = nullptr;
     host_materials.clear();
-    materials_recorded = false;
   }
   void free_paths() {
-    if (recorded)
-      retired.push_back(memory);
-    else
-      cudaFree(memory);
+    kept.give_up(memory, recorded);
     memory = nullptr;
     B = PathBuffers{};
-    recorded = false;
     capacity = 0;
   }
   // Places B's buffers for C paths from `base` on; returns their bytes.
@@ -114,7 +102,6 @@ struct PathScratch {
   }
   ~PathScratch() {
     cudaFree(memory);
-    for (void* m : retired) cudaFree(m);
     cudaFree(materials);
     cudaFree(counts);
     cudaFree(d_rgb);
@@ -127,15 +114,6 @@ void destroy_path_scratch(PathScratch* p) { delete p; }
 static int pfail(int code, const std::string& m) {
   set_error(m);
   return code;
-}
-
-static bool recording(cudaStream_t st) {
-  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
-  if (!st || cudaStreamIsCapturing(st, &c) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  return c == cudaStreamCaptureStatusActive;
 }
 
 static int path_prepare(Scene* s, const rq_path_params* p, PathParams& P, long long& total,

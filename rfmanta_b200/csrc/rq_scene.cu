@@ -42,6 +42,15 @@ cudaError_t device_alloc(void** p, size_t bytes) {
   return cudaMalloc(p, bytes);
 }
 
+bool recording(cudaStream_t st) {
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  if (!st || cudaStreamIsCapturing(st, &c) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return c == cudaStreamCaptureStatusActive;
+}
+
 static int fail(int code, const std::string& msg) {
   set_error(msg);
   return code;

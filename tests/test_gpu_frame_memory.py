@@ -81,3 +81,40 @@ def test_frames_after_failed_allocations(kind):
         assert np.array_equal(_bits(render(b, sc)), _bits(want))
     assert failed >= 2
     b.close()
+
+
+@pytest.mark.parametrize("kind", list(KINDS))
+def test_recorded_frames_keep_what_they_hold(kind):
+    """A frame recorded into a CUDA graph replays after frames with other tables and
+    larger ones."""
+    import torch
+    make, render = KINDS[kind]
+    sc = make()
+    b = _built(sc.mesh)
+    want = render(b, sc)
+    n = sc.xres * sc.yres
+    rgb = torch.zeros(3 * n, device="cuda")
+    t = torch.zeros(n, device="cuda")
+    prim = torch.zeros(n, dtype=torch.int32, device="cuda")
+    p = {"whitted": lambda: b.whitted_params(sc),
+         "supersampled": lambda: b.frame_params(sc, sc.mesh.materials),
+         "path": lambda: b.path_params(sc)}[kind]()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        st = torch.cuda.current_stream().cuda_stream
+        if kind == "whitted":
+            b.render_whitted_device(p, rgb.data_ptr(), t.data_ptr(), prim.data_ptr(), 0, st)
+        elif kind == "supersampled":
+            b.render_frame_device(p, rgb.data_ptr(), 0, st)
+        else:
+            b.render_path_device(p, rgb.data_ptr(), 0, st)
+    for k in range(3):
+        render(b, _other_materials(make(60 + 40 * k, 48 + 40 * k), k))
+    junk = [torch.full((1 << 10,), 7.0, device="cuda") for _ in range(64)]
+    junk.append(torch.full((1 << 22,), 7.0, device="cuda"))
+    g.replay()
+    torch.cuda.synchronize()
+    assert np.array_equal(_bits(rgb.cpu().numpy().reshape(-1, 3)), _bits(want))
+    assert np.array_equal(_bits(render(b, make())), _bits(want))
+    del g, junk
+    b.close()
